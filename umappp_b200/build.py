@@ -3,8 +3,8 @@
 Usage: python -m umappp_b200.build [--force] [-j N]
 
 Per-file flags: the stages whose results must round exactly as the
-reference's -ffp-contract=off build (similarities, graph, sgd) are compiled
-with -fmad=false; host code is compiled with -ffp-contract=off.
+reference's -ffp-contract=off build (similarities, graph, sgd, sgd_lists) are
+compiled with -fmad=false; host code is compiled with -ffp-contract=off.
 """
 from __future__ import annotations
 
@@ -25,8 +25,8 @@ NVCC = os.environ.get("NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
                  "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "--expt-relaxed-constexpr"]
-NO_FMAD = {"similarities.cu", "graph.cu", "sgd.cu"}
-SOURCES = ["capi.cu", "memory.cu", "knn.cu", "knn_tc.cu", "knn_tc16.cu", "knn_tree.cu", "similarities.cu", "graph.cu", "spectral.cu", "sgd.cu", "adjoint.cu", "probe.cu",
+NO_FMAD = {"similarities.cu", "graph.cu", "sgd.cu", "sgd_lists.cu"}
+SOURCES = ["capi.cu", "memory.cu", "knn.cu", "knn_tc.cu", "knn_tc16.cu", "knn_tree.cu", "similarities.cu", "graph.cu", "spectral.cu", "sgd.cu", "sgd_lists.cu", "adjoint.cu", "probe.cu",
            "find_ab.cpp"]
 
 

@@ -497,8 +497,6 @@ void batch_pipeline(const std::vector<int32_t>& inst, size_t data_dim, const voi
     SgdEngine<T> engine;
     engine.setup(&ep, s);
     engine.set_instances(d_inst.get(), ninst);
-    engine.use_graphs = true;
-    engine.autotune = true;
     tm.end();
     float ms_sched = 0, ms_sgd = 0;
     engine.run(Y.get(), static_cast<int>(num_dim), 0, epochs, a, b, o.repulsion_strength, o.learning_rate,

@@ -109,6 +109,8 @@ void ws_release_cached();
 size_t ws_set_limit(size_t bytes);   // cap on bytes held (in use + cached), 0: none; returns the previous cap
 cudaEvent_t event_get();          // timing event from the pool
 void event_put(cudaEvent_t e);
+void* pinned_get();               // 64 bytes of pinned host memory from the pool
+void pinned_put(void* p);         // no device work may still write it
 cudaStream_t stream_get(bool high_priority = false);   // non-blocking stream of the current device
 void stream_put(cudaStream_t s);  // s must be idle
 
@@ -134,11 +136,11 @@ public:
     void allocate(size_t n, cudaStream_t s) {
         release();
         stream_ = s;
-        n_ = n;
         if (n > 0) {
             if (n > SIZE_MAX / sizeof(T)) fail(UMAPB_ERR_OVERFLOW, "device allocation size overflows");
             ptr_ = static_cast<T*>(ws_alloc(n * sizeof(T), s));
         }
+        n_ = n;   // a failed allocation leaves an empty array
     }
     // Grows to at least n elements (contents are not kept); never shrinks.
     void reserve(size_t n, cudaStream_t s) {

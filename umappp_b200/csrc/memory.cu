@@ -192,12 +192,38 @@ std::vector<cudaEvent_t>& timing_events() {
     static auto* v = new std::vector<cudaEvent_t>();
     return *v;
 }
+std::mutex g_pinned_mu;
+std::vector<void*>& spare_pinned() {
+    static auto* v = new std::vector<void*>();
+    return *v;
+}
 std::mutex g_stream_mu;
 std::vector<std::pair<int, cudaStream_t>>& spare_streams() {   // (device * 2 + high priority, stream)
     static auto* v = new std::vector<std::pair<int, cudaStream_t>>();
     return *v;
 }
 }  // namespace
+
+// Pinned words for values a device computes and the host waits for: 64-byte
+// slots of 4 KiB blocks.  The pool holds as many as were ever in use at once.
+void* pinned_get() {
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    auto& v = spare_pinned();
+    if (v.empty()) {
+        char* block = nullptr;
+        UMAPB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&block), 4096, cudaHostAllocPortable));
+        for (int i = 0; i < 64; ++i) v.push_back(block + 64 * i);
+    }
+    void* p = v.back();
+    v.pop_back();
+    return p;
+}
+
+void pinned_put(void* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    spare_pinned().push_back(p);
+}
 
 cudaEvent_t event_get() {
     {

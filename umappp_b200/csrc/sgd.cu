@@ -3,39 +3,28 @@
 // Rows.  The reference walks the heads in order and, for each head, its
 // firing edges in CSR order: an attractive step that moves head and tail,
 // then that edge's negative samples, which move the head only.  Here one
-// thread takes one head's whole row, in the same per-row order: it evaluates
-// the schedule of each edge of the row in the reference's exact Float_
-// arithmetic (this file is compiled with -fmad=false), and for each firing
-// edge takes the attractive step and the negative samples.  No event lists
-// are built: the schedule state (epoch_of_next_sample and
-// epoch_of_next_negative_sample) is advanced in place, edge by edge, by the
-// thread that owns the edge's row.
+// thread (or a group of lanes, for layouts of more than four dimensions) takes
+// one head's whole row in that order, from a flat list of the points the head
+// meets in this epoch, which sgd_lists.cu has worked out ahead for a window of
+// epochs: the schedule and the samples do not depend on the layout.  What is
+// left is the chain that does: gather a point, take its step, move the head.
 //
-// Concurrency.  All rows of an epoch run at once (one launch per epoch);
-// warps claim chunks of 32 rows from a per-epoch counter, in an order fixed
-// per run: rows by descending firing rate (sum of 1 / epochs_per_sample), so
-// that the hubs -- heads with hundreds of firing edges per epoch at a million
-// points, whose rows are the longest sequential chains -- start first.  A
-// row's head is kept in registers and its displacement is added to the
-// embedding (vector atomic add) after every 'publish_every' firing edges and
-// at the end of the row; tails move by vector atomic adds.  Measured on a
+// Concurrency.  All rows of an epoch run at once (one launch per epoch), in a
+// claim order fixed per epoch (epoch_order_kernel): chunks of rows of
+// neighbouring index, rows that would end last ahead of them.  A row's head is kept in registers and
+// its displacement is added to the embedding (vector atomic add) after every
+// firing edge; tails move by vector atomic adds.  Measured on a
 // 1,000,000-point mixture against the serial reference's edge cross-entropy:
 // splitting a hub's row into concurrently processed pieces, or publishing the
 // head's move only at the end of a long row, leaves the layout about 1-1.5 %
 // tighter than the reference's; whole rows with the head published after each
 // firing edge come within about 0.3 %.
-//
-// Negative samples come from Philox4x32-10 keyed by the seed with counter
-// (head, tail, epoch, block), so they do not depend on the launch shape or on
-// how epochs are split across run() calls.
 #include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cfloat>
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -47,7 +36,7 @@ namespace umapb {
 namespace {
 
 constexpr int SCHED_BLOCK = 256;
-constexpr int MAX_GENERIC_DIM = 64;
+constexpr int MAX_DIM = 64;
 
 template <typename T>
 struct FloatLimits;
@@ -120,702 +109,426 @@ __global__ void __launch_bounds__(SCHED_BLOCK) sched_totals_kernel(int64_t nnz, 
 
 // ------------------------------------------------------------ row order --
 
-// Hub rows: expected to fire at least HUB_RATE edges per epoch.
-constexpr int HUB_RATE = 128;
 // Rows per group of the claim order (row_order_key_kernel).
 constexpr int ORDER_GROUP = 4096;
+constexpr float RATE_UNIT = 256.0f;   // firing rates are summed as multiples of 1 / RATE_UNIT
 
-// Order key of each row, sorted ascending: hub rows (firing rate -- the sum
-// of 1 / epochs_per_sample over the row, the expected number of firing edges
-// per epoch -- at least hub_rate) first, heaviest first; then the other rows
-// in groups of 'group' consecutive indices, in index order of the groups and
-// by descending rate within a group.  Rows in flight together then come from
-// a narrow index range (the concurrency the layout's quality depends on),
-// while the 32 rows a warp takes at once have similar lengths.
+// Firing rate of each row -- the sum of 1 / epochs_per_sample, the expected
+// number of firing edges per epoch -- and their sum (in integers: the same
+// whatever the order of the additions).
 template <typename T>
-__global__ void row_order_key_kernel(int32_t n, const int64_t* __restrict__ ptr, const T* __restrict__ eps,
-                                     float hub_rate, int32_t group, uint64_t* __restrict__ key,
-                                     int32_t* __restrict__ row, int* __restrict__ nhub) {
-    int hubs = 0;
+__global__ void row_rate_kernel(int32_t n, const int64_t* __restrict__ ptr, const T* __restrict__ eps,
+                                float* __restrict__ rate, unsigned long long* __restrict__ total) {
+    unsigned long long sum = 0;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float r = 0.0f;
         for (int64_t j = ptr[i]; j < ptr[i + 1]; ++j) r += 1.0f / static_cast<float>(eps[j]);
-        const bool hub = r >= hub_rate;
-        hubs += hub;
-        const uint64_t g = hub ? 0ull : 1ull + static_cast<uint64_t>(i / group);
-        key[i] = (g << 32) | static_cast<uint64_t>(~__float_as_uint(r));   // r >= 0: bits order as values
-        row[i] = i;
+        rate[i] = r;
+        sum += static_cast<unsigned long long>(fminf(fmaxf(r, 0.0f), 1e9f) * RATE_UNIT);
     }
-    for (int o = 16; o > 0; o >>= 1) hubs += __shfl_xor_sync(0xffffffffu, hubs, o);
-    if ((threadIdx.x & 31) == 0 && hubs) atomicAdd(nhub, hubs);
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total, sum);
 }
 
-// The non-hub rows of one epoch in claim order: every chunk of ORDER_GROUP
-// consecutive positions of the run's order (hub rows left out) sorted by
-// descending number of edges that fire in this epoch -- counted by the
-// previous epoch's kernel while it scanned the rows (RowArgs::next_count) --,
-// equal counts (and counts of 255 or more) in the run's order (a stable sort).  A chunk keeps its
-// positions, so the rows in flight together still come from one index range,
-// while the 32 rows a warp takes fire the same number of edges (and rows that
-// fire none come last).
+// Order key of each row, sorted ascending: groups of 'group' consecutive
+// indices in index order, by descending rate within a group.  Rows in flight
+// together then come from a narrow index range (the concurrency the layout's
+// quality depends on), while the 32 rows a warp takes at once have similar
+// lengths.  A row so long that, started in its own group's turn, it would
+// still run when all other rows are done, goes to the last group from whose
+// turn it ends in time: 'lanes' rows run at once, each lane for total / lanes
+// in all, and group g starts after g / groups of that.  (Hubs are up to 50
+// times the mean length: one taken in the last group's turn would decide the
+// epoch's time.)
+__global__ void row_order_key_kernel(int32_t n, const float* __restrict__ rate,
+                                     const unsigned long long* __restrict__ total, int64_t lanes, int32_t group,
+                                     uint64_t* __restrict__ key, int32_t* __restrict__ row) {
+    const float span = static_cast<float>(static_cast<double>(*total) / (RATE_UNIT * static_cast<double>(lanes)));
+    const int32_t groups = (n - 1) / group + 1;
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float r = rate[i];
+        const float slack = span > 0.0f ? fminf(fmaxf(1.0f - r / span, 0.0f), 1.0f) : 1.0f;   // of the epoch, after which it must have started
+        const int32_t latest = static_cast<int32_t>(slack * static_cast<float>(groups));
+        const uint32_t g = static_cast<uint32_t>(min(i / group, latest));
+        key[i] = (static_cast<uint64_t>(g) << 32) | static_cast<uint64_t>(~__float_as_uint(fmaxf(r, 0.0f)));   // r >= 0: bits order as values
+        row[i] = i;
+    }
+}
+
+// Claim order of the epochs of a window (blockIdx.y): every chunk of
+// ORDER_GROUP consecutive positions of the run's order sorted by descending
+// number of entries in this epoch (equal counts, and counts of 4095 or more,
+// in the run's order: a stable sort).  A chunk keeps its positions, so the
+// rows in flight together still come from one index range, while the 32 rows
+// a warp takes have nearly equal lists (and rows without entries come last).
 constexpr int EPOCH_ORDER_THREADS = 512;
 constexpr int EPOCH_ORDER_ITEMS = ORDER_GROUP / EPOCH_ORDER_THREADS;
 __global__ void __launch_bounds__(EPOCH_ORDER_THREADS)
-    epoch_bulk_order_kernel(const int32_t* __restrict__ run_order, int32_t nbulk, const uint16_t* __restrict__ count,
-                            int32_t* __restrict__ bulk) {
+    epoch_order_kernel(const int32_t* __restrict__ run_order, int32_t n, bool sort, const ListSpan* __restrict__ span,
+                       RowTask* __restrict__ tasks) {
     using Sort = cub::BlockRadixSort<uint32_t, EPOCH_ORDER_THREADS, EPOCH_ORDER_ITEMS, int32_t>;
     __shared__ typename Sort::TempStorage tmp;
+    span += static_cast<int64_t>(blockIdx.y) * n;
+    tasks += static_cast<int64_t>(blockIdx.y) * n;
     const int64_t first = static_cast<int64_t>(blockIdx.x) * ORDER_GROUP + threadIdx.x * EPOCH_ORDER_ITEMS;
     uint32_t key[EPOCH_ORDER_ITEMS];
     int32_t row[EPOCH_ORDER_ITEMS];
 #pragma unroll
     for (int i = 0; i < EPOCH_ORDER_ITEMS; ++i) {   // blocked: item rank = position in the chunk
         const int64_t pos = first + i;
-        row[i] = pos < nbulk ? run_order[pos] : -1;
-        // descending count, capped at 255 (non-hub rows fire fewer edges than
-        // that), in 8 bits; past the end: 256, last
-        key[i] = pos < nbulk ? 255u - min(static_cast<uint32_t>(count[row[i]]), 255u) : 256u;
+        row[i] = pos < n ? run_order[pos] : -1;
+        key[i] = 4095u;   // past the end: last (and the stable sort keeps them behind rows without entries)
+        if (pos < n) {
+            const ListSpan sp = span[row[i]];
+            key[i] = 4095u - min(sp.end - sp.start8 * LIST_ALIGN, 4095u);
+        }
     }
-    Sort(tmp).Sort(key, row, 0, 9);
+    if (sort) Sort(tmp).Sort(key, row, 0, 12);
 #pragma unroll
-    for (int i = 0; i < EPOCH_ORDER_ITEMS; ++i)
-        if (first + i < nbulk) bulk[first + i] = row[i];
+    for (int i = 0; i < EPOCH_ORDER_ITEMS; ++i) {
+        if (first + i < n) {
+            const ListSpan sp = span[row[i]];
+            *reinterpret_cast<int4*>(tasks + first + i) =
+                make_int4(row[i], static_cast<int>(sp.start8), static_cast<int>(sp.end - sp.start8 * LIST_ALIGN), 0);
+        }
+    }
 }
 
 // ---------------------------------------------------------- epoch kernels --
 
 template <typename T>
-struct SgdParams {
+struct StepParams {
     T a, b;
     T neg2ab;      // -2ab
     T gamma2b;     // 2 gamma b
     T alpha;
-    T rate;        // negative_sample_rate in Float_
-    T epoch;       // the epoch as Float_
-    uint32_t k0, k1;
-    uint32_t epoch_u;
-    int32_t n;
-    int32_t publish_every;
-    // Independent instances laid out one after another (batched runs):
-    // instance i owns observations [inst_start[i], inst_start[i + 1]) and
-    // draws its negative samples there.  num_inst <= 1: one instance of n.
-    const int32_t* inst_start;
-    int32_t num_inst;
 };
 
-// The rows of one epoch and where they are claimed from.
-template <typename T>
-struct RowArgs {
-    const int32_t* order;      // rows in processing order
-    int32_t nrows;
-    const int64_t* ptr;
-    const int32_t* targets;
-    const T* eps;
-    T* enext;
-    T* enneg;
-    int* counter;              // claims so far in this epoch: [0] hub rows (or row groups), [1] other rows
-    unsigned long long* totals;   // optional: [firing edges, negative samples drawn] of this epoch
-    int32_t nhub;              // 2-d kernel: order[0, nhub) are hub rows, one warp each
-    const int32_t* bulk;       // 2-d kernel: the other rows in this epoch's claim order (null: order + nhub)
-    uint16_t* next_count;      // 2-d kernel, optional: receives each non-hub row's firing edges in the next epoch
-};
-
-// Observation range [base, base + size) of the instance that owns h.
-template <typename T>
-__device__ __forceinline__ void instance_range(int32_t h, const SgdParams<T>& p, int32_t& base, uint32_t& size) {
-    if (p.num_inst <= 1) {
-        base = 0;
-        size = static_cast<uint32_t>(p.n);
-        return;
-    }
-    int lo = 0, hi = p.num_inst - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (p.inst_start[mid] <= h) lo = mid; else hi = mid - 1;
-    }
-    base = p.inst_start[lo];
-    size = static_cast<uint32_t>(p.inst_start[lo + 1] - base);
+// clamp to [-4, 4] and floor to epsilon; a NaN gradient stays NaN, a NaN
+// distance takes the floor, as the reference's comparisons have it
+__device__ __forceinline__ float clamp4(float g) {
+    asm("max.NaN.f32 %0, %0, 0fC0800000;\n\tmin.NaN.f32 %0, %0, 0f40800000;" : "+f"(g));
+    return g;
 }
-
-// Counter-based negative-sample stream of one firing edge (Philox4x32-7).
-struct NegStream {
-    uint32_t c0, c1, c2, c3, k0, k1;
-    Philox4 buf;
-    int used;
-    __device__ __forceinline__ NegStream(uint32_t h, uint32_t t, uint32_t epoch, uint32_t key0, uint32_t key1)
-        : c0(h), c1(t), c2(epoch), c3(0), k0(key0), k1(key1), used(4) {}
-    __device__ __forceinline__ uint32_t next() {
-        if (used == 4) {
-            // 7 rounds: the fewest for which Salmon et al. found Philox4x32
-            // free of BigCrush failures; negative samples only need uniform,
-            // independent indices, and the rounds are a tenth of an edge's work
-            buf = philox4x32<7>(c0, c1, c2, c3++, k0, k1);
-            used = 0;
-        }
-        // a select chain rather than buf.v[used]: a dynamically indexed array would live in local memory
-        const uint32_t v = used == 0 ? buf.v[0] : used == 1 ? buf.v[1] : used == 2 ? buf.v[2] : buf.v[3];
-        ++used;
-        return v;
-    }
-    // Exactly uniform integer in [0, n) (Lemire, "Fast random integer generation
-    // in an interval", ACM TOMACS 2019): multiply-shift with rejection.
-    __device__ __forceinline__ int32_t bounded(uint32_t n) {
-        uint64_t m = static_cast<uint64_t>(next()) * n;
-        uint32_t l = static_cast<uint32_t>(m);
-        if (l < n) {
-            const uint32_t thr = (0u - n) % n;
-            while (l < thr) {
-                m = static_cast<uint64_t>(next()) * n;
-                l = static_cast<uint32_t>(m);
-            }
-        }
-        return static_cast<int32_t>(m >> 32);
-    }
-};
-
-template <typename T>
-__device__ __forceinline__ T clamp4(T g) {
-    g = (g < T(-4)) ? T(-4) : g;
-    return (T(4) < g) ? T(4) : g;
+__device__ __forceinline__ double clamp4(double g) {
+    g = (g < -4.0) ? -4.0 : g;
+    return (4.0 < g) ? 4.0 : g;
 }
-
-// The step coefficients, optimize_layout.hpp:147-149 (attractive) and
-// :170-171 (repulsive), from the edge derivatives shared with the adjoint
-// (umap_grad.cuh): attractive = -2 dA/dd2, repulsive = -2 gamma dR/dd2 with
-// eps = 0.001.  FP32 layouts use the hardware-approximated power (__powf, an
-// exp2 of b log2 x in the special-function unit) and divide (__fdividef): the
-// step is stochastic and clamped, and the layout's cross-entropy was measured
-// unchanged with libm's powf and IEEE division at a million points.
-template <typename T>
-__device__ __forceinline__ T attract_coef(T d2, const SgdParams<T>& p) {
-    return attract_dd2<std::is_same<T, float>::value>(d2, p.a, p.b, p.neg2ab);
-}
-
-template <typename T>
-__device__ __forceinline__ T repulse_coef(T d2, const SgdParams<T>& p) {
-    return repulse_dd2<std::is_same<T, float>::value>(d2, p.a, p.b, p.gamma2b, T(0.001));
-}
-
-__device__ __forceinline__ float attract_coef_fast(float d2, const SgdParams<float>& p) { return attract_coef(d2, p); }
-__device__ __forceinline__ float repulse_coef_fast(float d2, const SgdParams<float>& p) { return repulse_coef(d2, p); }
-
-template <typename T>
-__device__ __forceinline__ T floor_eps(T d2) {
-    const T e = FloatLimits<T>::epsilon();
+__device__ __forceinline__ float floor_eps(float d2) { return fmaxf(d2, FloatLimits<float>::epsilon()); }
+__device__ __forceinline__ double floor_eps(double d2) {
+    const double e = FloatLimits<double>::epsilon();
     return (e < d2) ? d2 : e;
 }
 
-// Next firing edge of a row at or after j (r1: none).
+// The gradient of one step (before the clamp) along every coordinate
+// difference, optimize_layout.hpp:147-155 (attractive) and :170-176
+// (repulsive): one power, one divide.
+template <int NC>
+__device__ __forceinline__ void step_gradient(double d2, bool attract, const double (&diff)[NC],
+                                              const StepParams<double>& p, double (&g)[NC]) {
+    const double q = pow(d2, p.b);
+    const double c = (attract ? p.neg2ab * q : p.gamma2b) / ((attract ? d2 : 0.001 + d2) * (p.a * q + 1.0));
+#pragma unroll
+    for (int j = 0; j < NC; ++j) g[j] = c * diff[j];
+}
+
+// FP32 layouts use the special-function unit's approximations (2^(b log2 d2)
+// and a reciprocal; d2 is at least FLT_EPSILON, so no operand is subnormal):
+// the step is stochastic and clamped, and the layout's cross-entropy was
+// measured unchanged with libm's powf and IEEE division at a million points.
+// A row is one chain of these steps, so the products are grouped to shorten
+// it: after the power one fused multiply-add, the reciprocal and a product.
+template <int NC>
+__device__ __forceinline__ void step_gradient(float d2, bool attract, const float (&diff)[NC],
+                                              const StepParams<float>& p, float (&g)[NC]) {
+    float l, q, r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(d2));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(l * p.b));
+    const float e2 = attract ? d2 : 0.001f + d2, num = attract ? p.neg2ab : p.gamma2b;
+    const float den = __fmaf_rn(e2 * p.a, q, e2);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+    const float c = num * (attract ? q : 1.0f) * r;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) g[j] = c * diff[j];
+}
+
+// The transform's coefficients: the two written out apart (umap_grad.cuh).
 template <typename T>
-__device__ __forceinline__ int64_t next_firing(const T* __restrict__ enext, int64_t j, int64_t r1, T epoch) {
-    while (j < r1 && enext[j] > epoch) ++j;
-    return j;
+__device__ __forceinline__ T transform_coef(T d2, bool attract, const StepParams<T>& p) {
+    constexpr bool fast = std::is_same<T, float>::value;
+    return attract ? attract_dd2<fast>(d2, p.a, p.b, p.neg2ab) : repulse_dd2<fast>(d2, p.a, p.b, p.gamma2b, T(0.001));
 }
 
-// The warp's next chunk of 32 rows (all lanes get the same base).
-__device__ __forceinline__ int32_t claim_rows(int* counter) {
-    int32_t base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(counter, 32);
-    return __shfl_sync(0xffffffffu, base, 0);
-}
-
-__device__ __forceinline__ void add_totals(unsigned long long* totals, unsigned long long fired,
-                                           unsigned long long drawn) {
-    if (!totals) return;
-    for (int o = 16; o > 0; o >>= 1) {
-        fired += __shfl_xor_sync(0xffffffffu, fired, o);
-        drawn += __shfl_xor_sync(0xffffffffu, drawn, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&totals[0], fired);
-        atomicAdd(&totals[1], drawn);
-    }
-}
+// x + y z: fused for float layouts, separately rounded for double ones
+__device__ __forceinline__ float madd(float x, float y, float z) { return __fmaf_rn(y, z, x); }
+__device__ __forceinline__ double madd(double x, double y, double z) { return x + y * z; }
 
 // Coherent device-scope load: ordered after this thread's own earlier atomic
 // adds to the same address (per-location coherence), so a head re-read after
 // its own publication sees it, plus whatever other threads have added.
-__device__ __forceinline__ float2 ld_relaxed_f2(const float2* q) {
-    float2 v;
-    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(q) : "memory");
+__device__ __forceinline__ float ld_relaxed(const float* q) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(q) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_relaxed(const double* q) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(q) : "memory");
     return v;
 }
 
-// 2-d FP32 rows.  Work units, claimed by warps in order: first the hub rows
-// (one row per warp), then the other rows, 32 per warp (one per lane).
-constexpr int BULK_CHUNK = 8;    // edges of a row whose schedule state a lane loads at once
-
-// A row's schedule state, read BULK_CHUNK edges at a time into registers
-// (the next window's loads in flight while the current one is used), and the
-// row's firing edges found in it in order.
-__device__ __forceinline__ void cp_async4(float* dst_shared, const float* src, bool valid) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst_shared));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+// Vector and scalar adds to global memory where e is negative (predicated, not
+// branched over: a chain of steps then stays one straight piece of code).
+__device__ __forceinline__ void red_if_negative(int32_t e, float* q, float x) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %0, 0;\n\t@p red.relaxed.gpu.global.add.f32 [%1], %2;\n\t}" ::"r"(e),
+                 "l"(q), "f"(x));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// A lane's scan of its row's epoch_of_next_sample, BULK_CHUNK edges at a
-// time, through two windows in shared memory (the lane's column of its warp's
-// slab, [buffer][edge][lane]: conflict-free): the next window is copied
-// asynchronously (cp.async) while the current one is used.
-struct RowScan {
-    int64_t cb, nb, r1;        // current window's first edge, next window's first edge, row end
-    float* w;                  // this lane's column: w[(buffer * BULK_CHUNK + q) * 32]
-    unsigned cm;               // firing edges of the current window not yet taken
-    int cur;                   // buffer of the current window
-    int n1;                    // edges seen so far that fire at the next epoch (their new state counted
-                               // by lane_row_step for the ones that fire now)
-    __device__ __forceinline__ void load(int buf, const float* __restrict__ enext, int64_t b) {
-#pragma unroll
-        for (int q = 0; q < BULK_CHUNK; ++q) {
-            const bool ok = b + q < r1;
-            cp_async4(&w[(buf * BULK_CHUNK + q) * 32], ok ? enext + b + q : enext, ok);
-        }
-        cp_async_commit();
-    }
-    __device__ __forceinline__ unsigned fire_mask(int buf, int64_t b, float ef) {
-        // b < r1 here; edges past the row's end are masked off
-        unsigned m = 0, m1 = 0;
-        const float ef1 = ef + 1.0f;   // the next epoch (an integer: exact)
-#pragma unroll
-        for (int q = 0; q < BULK_CHUNK; ++q) {
-            const float v = w[(buf * BULK_CHUNK + q) * 32];
-            m |= (v <= ef ? 1u : 0u) << q;
-            m1 |= (v <= ef1 ? 1u : 0u) << q;
-        }
-        const int64_t left = r1 - b;
-        const unsigned valid = left >= BULK_CHUNK ? (1u << BULK_CHUNK) - 1u : (1u << static_cast<int>(left)) - 1u;
-        m &= valid;
-        n1 += __popc(m1 & valid) - __popc(m);   // fire at the next epoch, not at this one
-        return m;
-    }
-    __device__ __forceinline__ void start(float* column, const float* __restrict__ enext, int64_t j0, int64_t end,
-                                          float ef) {
-        // the lane's previous row may have left a window copy in flight into
-        // these buffers: let it land before they are refilled
-        cp_async_wait<0>();
-        w = column;
-        r1 = end;
-        cb = j0;
-        nb = j0 + BULK_CHUNK;
-        cur = 0;
-        n1 = 0;
-        load(0, enext, cb);
-        load(1, enext, nb);
-        cp_async_wait<1>();
-        cm = fire_mask(0, cb, ef);
-    }
-    // Next firing edge (false: none left); en = its epoch_of_next_sample.
-    __device__ __forceinline__ bool next(const float* __restrict__ enext, float ef, int64_t& j, float& en) {
-        while (cm == 0) {
-            if (nb >= r1) return false;
-            cb = nb;
-            cur ^= 1;
-            cp_async_wait<0>();
-            cm = fire_mask(cur, cb, ef);
-            nb += BULK_CHUNK;
-            load(cur ^ 1, enext, nb);
-        }
-        const int q = __ffs(cm) - 1;
-        cm &= cm - 1;
-        j = cb + q;
-        en = w[(cur * BULK_CHUNK + q) * 32];
-        return true;
-    }
-};
-
-// One firing edge of a lane's row, with its target and schedule state.
-struct RowEdge {
-    int64_t j;
-    float en, ep, enn;
-    int32_t t;
-};
-
-// A lane's current row: its scan, the firing edge at hand (cur: state loaded
-// two steps ago), the one after it (nxt: state loads in flight) and its
-// instance's range for negative samples.
-struct LaneRow {
-    int32_t h;       // -1: none
-    float hx, hy;    // the head, when it is not re-read (FRESH = false)
-    int32_t nbase;
-    uint32_t nsize;
-    bool has_nxt;
-    RowEdge cur, nxt;
-    RowScan sc;
-};
-
-// Finds the row's next firing edge and issues its state loads.
-__device__ __forceinline__ bool lane_row_fetch(LaneRow& L, RowEdge& e, const RowArgs<float>& r, float ef) {
-    if (!L.sc.next(r.enext, ef, e.j, e.en)) return false;
-    e.t = r.targets[e.j];
-    e.ep = r.eps[e.j];
-    e.enn = r.enneg[e.j];
-    return true;
+__device__ __forceinline__ void red_if_negative(int32_t e, double* q, double x) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %0, 0;\n\t@p red.relaxed.gpu.global.add.f64 [%1], %2;\n\t}" ::"r"(e),
+                 "l"(q), "d"(x));
+}
+__device__ __forceinline__ void red_if_negative(int32_t e, float* q, float x, float y) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %0, 0;\n\t"
+                 "@p red.relaxed.gpu.global.add.v2.f32 [%1], {%2, %3};\n\t}" ::"r"(e),
+                 "l"(q), "f"(x), "f"(y));
+}
+__device__ __forceinline__ void red_if_negative(int32_t e, float* q, float x, float y, float z, float u) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %0, 0;\n\t"
+                 "@p red.relaxed.gpu.global.add.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"(e),
+                 "l"(q), "f"(x), "f"(y), "f"(z), "f"(u));
 }
 
-// Starts row h on a lane: false when the row fires no edge this epoch.
-template <typename P>
-__device__ __forceinline__ bool lane_row_start(LaneRow& L, int32_t h, const RowArgs<float>& r, const float2* Y,
-                                               const P& p, float* column) {
-    const float ef = p.epoch;
-    const int64_t j0 = r.ptr[h], r1 = r.ptr[h + 1];
-    if (j0 >= r1) {
-        if (r.next_count) r.next_count[h] = 0;
-        return false;
-    }
-    L.sc.start(column, r.enext, j0, r1, ef);
-    if (!lane_row_fetch(L, L.cur, r, ef)) {   // the whole row scanned: nothing fires now
-        if (r.next_count) r.next_count[h] = static_cast<uint16_t>(min(L.sc.n1, 65535));
-        return false;
-    }
-    L.has_nxt = lane_row_fetch(L, L.nxt, r, ef);
-    L.h = h;
-    const float2 y0 = __ldcg(&Y[h]);
-    L.hx = y0.x;
-    L.hy = y0.y;
-    instance_range(h, p, L.nbase, L.nsize);
-    return true;
-}
-
-// One firing edge of a lane's row.  The head (re-read: it sees the pulls of
-// other rows' attractive steps), the tail and the first NB negative samples
-// are gathered together -- the negative-sample indices do not depend on the
-// layout; while they are in flight the schedule step is written and the
-// state loads of the firing edge after the next one are issued (so an edge's
-// gathers never wait for its own state); then the updates are applied in the
-// reference's order and the head's move is published.  Returns false when
-// the row has no firing edge left.
-template <int NB, bool FRESH>
-__device__ __forceinline__ bool lane_row_step(LaneRow& L, const RowArgs<float>& r, float2* __restrict__ Y,
-                                              const SgdParams<float>& p, unsigned long long& fired,
-                                              unsigned long long& drawn) {
-    const float ef = p.epoch;
-    const int32_t h = L.h, t = L.cur.t;
-    const float2 yh = FRESH ? ld_relaxed_f2(&Y[h]) : make_float2(L.hx, L.hy);
-    const float2 yt = __ldcg(&Y[t]);
-    const float epns = L.cur.ep / p.rate;   // optimize_layout.hpp:160-161
-    const int nn = static_cast<int>((ef - L.cur.enn) / epns);
-    int remaining = nn > 0 ? nn : 0;         // a negative count draws nothing, as in the reference's loop
-    NegStream rng(static_cast<uint32_t>(h), static_cast<uint32_t>(t), p.epoch_u, p.k0, p.k1);
-    int m = remaining < NB ? remaining : NB;
-    int32_t ks[NB];
-    float2 yk[NB];
+// A point as its lane group holds it: G lanes with NC coordinates each, lane g
+// of the group the coordinates g, g + G, ...  G = 1: the whole point (dim = NC),
+// read and added to as vectors where its size allows (the embedding is
+// aligned to them, SgdEngine::run).
+template <typename T, int NC, int G>
+struct Point {
+    T v[NC];
+    __device__ __forceinline__ void load(const T* __restrict__ Y, int32_t k, int dim) {
+        if constexpr (G == 1 && NC == 2 && sizeof(T) == 4) {
+            const float2 q = __ldcg(reinterpret_cast<const float2*>(Y) + k);
+            v[0] = q.x, v[1] = q.y;
+        } else if constexpr (G == 1 && NC == 4 && sizeof(T) == 4) {
+            const float4 q = __ldcg(reinterpret_cast<const float4*>(Y) + k);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else if constexpr (G == 1 && NC % 2 == 0) {
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        if (b < m) {
-            ks[b] = L.nbase + rng.bounded(L.nsize);
-            yk[b] = __ldcg(&Y[ks[b]]);
-        }
-    }
-    const float en_new = L.cur.en + L.cur.ep;                 // :178-179
-    r.enext[L.cur.j] = en_new;
-    r.enneg[L.cur.j] = L.cur.enn + static_cast<float>(nn) * epns;
-    L.sc.n1 += en_new <= ef + 1.0f ? 1 : 0;
-    ++fired;
-    drawn += remaining;
-    // rotate: nxt becomes cur; fetch the one after
-    const bool more = L.has_nxt;
-    if (more) {
-        L.cur = L.nxt;
-        L.has_nxt = lane_row_fetch(L, L.nxt, r, ef);
-    }
-    float hx = yh.x, hy = yh.y;
-    {   // attractive step (:145-155)
-        const float dx = hx - yt.x, dy = hy - yt.y;
-        const float d2 = floor_eps(__fmaf_rn(dx, dx, dy * dy));
-        const float cf = attract_coef_fast(d2, p);
-        const float gx = p.alpha * clamp4(cf * dx);
-        const float gy = p.alpha * clamp4(cf * dy);
-        hx += gx;
-        hy += gy;
-        atomicAdd(&Y[t], make_float2(-gx, -gy));
-    }
-    while (true) {   // negative samples (:157-176)
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            if (b < m && ks[b] != h) {
-                const float dx = hx - yk[b].x, dy = hy - yk[b].y;
-                const float d2 = floor_eps(__fmaf_rn(dx, dx, dy * dy));
-                const float cf = repulse_coef_fast(d2, p);
-                hx = __fmaf_rn(p.alpha, clamp4(cf * dx), hx);
-                hy = __fmaf_rn(p.alpha, clamp4(cf * dy), hy);
+            for (int j = 0; j < NC / 2; ++j) {
+                const double2 q = __ldcg(reinterpret_cast<const double2*>(Y) + static_cast<int64_t>(k) * (NC / 2) + j);
+                v[2 * j] = q.x, v[2 * j + 1] = q.y;
             }
+        } else {
+            each(Y, k, dim, [](T& x, const T* q) { x = __ldcg(q); });
         }
-        remaining -= m;
-        if (remaining <= 0) break;
-        m = remaining < NB ? remaining : NB;
+    }
+    __device__ __forceinline__ void reload(const T* Y, int32_t k, int dim) {
+        each(Y, k, dim, [](T& x, const T* q) { x = ld_relaxed(q); });
+    }
+    // Adds the coordinates to point k where e is negative.
+    __device__ __forceinline__ void add_if_negative(int32_t e, T* __restrict__ Y, int32_t k, int dim) const {
+        T* q = Y + static_cast<int64_t>(k) * (G == 1 ? NC : dim);
+        if constexpr (G == 1 && NC == 2 && sizeof(T) == 4) {
+            red_if_negative(e, q, v[0], v[1]);
+        } else if constexpr (G == 1 && NC == 4 && sizeof(T) == 4) {
+            red_if_negative(e, q, v[0], v[1], v[2], v[3]);
+        } else {
+            const int g = threadIdx.x & (G - 1);
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            if (b < m) {
-                ks[b] = L.nbase + rng.bounded(L.nsize);
-                yk[b] = __ldcg(&Y[ks[b]]);
+            for (int j = 0; j < NC; ++j) {
+                const int c = g + j * G;
+                red_if_negative(G == 1 || c < dim ? e : 0, q + c, v[j]);
             }
         }
     }
-    atomicAdd(&Y[h], make_float2(hx - yh.x, hy - yh.y));
-    L.hx = hx;
-    L.hy = hy;
-    // the row's last firing edge: every window has been scanned
-    if (!more && r.next_count) r.next_count[h] = static_cast<uint16_t>(min(L.sc.n1, 65535));
-    return more;
-}
-
-// Gathered operands of one firing edge of a hub row (shared memory).
-template <int NB>
-struct HubEvent {
-    float2 yt;
-    float2 yk[NB];
-    int32_t ks[NB];
-    int32_t t;
-    int32_t nn;
+    template <class F>
+    __device__ __forceinline__ void each(const T* Y, int32_t k, int dim, F f) {
+        const T* row = Y + static_cast<int64_t>(k) * (G == 1 ? NC : dim);
+        const int g = threadIdx.x & (G - 1);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            if (G == 1) f(v[j], row + j);
+            else if (g + j * G < dim) f(v[j], row + g + j * G);
+            else v[j] = T(0);
+        }
+    }
 };
 
-// A hub row, by a whole warp: the lanes take 32 edges at a time -- schedule
-// step, tail and first NB negative samples gathered into shared memory, all
-// in parallel -- and lane 0 then applies the chunk's firing edges in order,
-// publishing the head's move after each edge.  Lane 0 re-reads the head at
-// the start of every chunk (the value arrives while the chunk is gathered) and
-// at the chunk's end takes it, plus the chunk's own moves, as the head: the
-// pulls of other rows' attractive steps on the hub are seen a chunk late.
-template <int NB>
-__device__ __forceinline__ void hub_row(int32_t h, const RowArgs<float>& r, float2* __restrict__ Y,
-                                        const SgdParams<float>& p, HubEvent<NB>* __restrict__ ev,
-                                        unsigned long long& fired, unsigned long long& drawn) {
+// CH entries of a list, from an address aligned to them.
+template <int CH>
+struct Entries {
+    int32_t e[CH];
+    __device__ __forceinline__ void load(const int32_t* __restrict__ p) {
+#pragma unroll
+        for (int i = 0; i < CH; i += 4) {
+            const int4 q = __ldg(reinterpret_cast<const int4*>(p + i));
+            e[i] = q.x, e[i + 1] = q.y, e[i + 2] = q.z, e[i + 3] = q.w;
+        }
+    }
+    __device__ __forceinline__ int32_t point(int i) const { return e[i] & INT32_MAX; }
+};
+
+// The first entries of a row's list, read ahead.
+template <int CH>
+struct ListHead {
+    const int32_t* p;
+    uint32_t cnt, chunks;
+    Entries<CH> e0, e1;
+    __device__ __forceinline__ void load(const int32_t* __restrict__ list, uint32_t start8, uint32_t count) {
+        p = list + static_cast<int64_t>(start8) * LIST_ALIGN;
+        cnt = count;
+        chunks = (count + CH - 1) / CH;
+        if (chunks) e0.load(p);
+        if (chunks > 1) e1.load(p + CH);
+    }
+};
+
+// One row's list applied to its head, CH entries at a time: while CH steps
+// run, the points of the next CH are gathered and the entries after those
+// read.  The head's move is published at every firing edge, together with the
+// edge's own pull on its tail, and a long row's head re-read after every 256
+// entries, with the other rows' pulls on it.  (Published after every 8 entries
+// instead, a step costs 151 cycles against 200, but the layout's cross-entropy
+// at 100,000 points is 2.9 % above the reference's; as it is, 0.05 %.)
+// What bounds a row is the chain of its steps -- some 100 cycles each of
+// dependent arithmetic -- so the steps are straight code of few instructions:
+// the lists are padded with the head itself, and an entry equal to the head
+// (padding, or a sample that hit it) takes a step of rate 0.
+// FIXED (transform): only the head moves, it is not published, and the list's
+// padding is not read.  A row without entries does nothing.
+template <typename T, int NC, int G, int CH, bool FIXED>
+struct RowWalk {
+    Point<T, NC, G>& head;
+    const int32_t h;
+    const ListHead<CH>& l;
+    T* __restrict__ Y;
+    const int dim;
+    const StepParams<T>& p;
+    Point<T, NC, G> pub;
+
+    __device__ __forceinline__ void gather(Point<T, NC, G> (&y)[CH], const Entries<CH>& e, uint32_t c) {
+        if (c < l.chunks) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i)
+                if (!FIXED || c * CH + i < l.cnt) y[i].load(Y, e.point(i), dim);
+        }
+    }
+    // Where e is negative.
+    __device__ __forceinline__ void publish(int32_t e) {
+        Point<T, NC, G> d;
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            d.v[j] = head.v[j] - pub.v[j];
+            pub.v[j] = e < 0 ? head.v[j] : pub.v[j];
+        }
+        d.add_if_negative(e, Y, h, dim);
+    }
+    // Chunk c's entries e at the points y; chunk c + 1 is gathered from en to
+    // yn, and chunk c + 2 takes the place of e.
+    __device__ __forceinline__ void chunk(uint32_t c, Entries<CH>& e, const Point<T, NC, G> (&y)[CH],
+                                          const Entries<CH>& en, Point<T, NC, G> (&yn)[CH]) {
+        gather(yn, en, c + 1);
+        Entries<CH> far;
+        if (c + 2 < l.chunks) far.load(l.p + (c + 2) * CH);
+        if (!FIXED && c > 0 && c % (256 / CH) == 0) {
+            publish(-1);
+            head.reload(Y, h, dim);
+            pub = head;
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const bool attract = e.e[i] < 0;
+            T diff[NC], d2 = 0, grad[NC];
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                diff[j] = head.v[j] - y[i].v[j];
+                d2 = FIXED ? d2 + diff[j] * diff[j] : madd(d2, diff[j], diff[j]);
+            }
+            if constexpr (G > 1) {   // the group's lanes share the row
+                const unsigned group = (G == 32 ? 0xffffffffu : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) d2 += __shfl_xor_sync(group, d2, o, G);
+            }
+            d2 = floor_eps(d2);
+            if constexpr (FIXED) {
+                const T cf = transform_coef(d2, attract, p);
+#pragma unroll
+                for (int j = 0; j < NC; ++j) grad[j] = cf * diff[j];
+            } else {
+                step_gradient(d2, attract, diff, p, grad);
+            }
+            const T rate = (FIXED ? c * CH + i < l.cnt : e.e[i] != h) ? p.alpha : T(0);
+            Point<T, NC, G> pull;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const T g = clamp4(grad[j]);
+                head.v[j] = FIXED ? head.v[j] + rate * g : madd(head.v[j], rate, g);
+                pull.v[j] = -(rate * g);
+            }
+            if (!FIXED) {
+                pull.add_if_negative(e.e[i], Y, e.point(i), dim);
+                publish(e.e[i]);
+            }
+        }
+        e = far;
+    }
+    __device__ __forceinline__ void run() {
+        Entries<CH> e0 = l.e0, e1 = l.e1;
+        Point<T, NC, G> y0[CH], y1[CH];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) y0[i] = y1[i] = head;
+        gather(y0, e0, 0);
+        for (uint32_t c = 0; c < l.chunks; c += 2) {
+            chunk(c, e0, y0, e1, y1);
+            if (c + 1 < l.chunks) chunk(c + 1, e1, y1, e0, y0);
+        }
+        if (!FIXED && l.chunks) publish(-1);
+    }
+};
+
+template <typename T, int NC, int G, int CH, bool FIXED>
+__device__ __forceinline__ void walk_row(Point<T, NC, G>& head, int32_t h, const ListHead<CH>& l, T* __restrict__ Y,
+                                         int dim, const StepParams<T>& p) {
+    RowWalk<T, NC, G, CH, FIXED> w{head, h, l, Y, dim, p, head};
+    w.run();
+}
+
+constexpr int ROW_BLOCK = 64;
+constexpr int ROW_BLOCKS = 4;   // resident per SM
+
+// One epoch: warps claim 32 / G rows at a time in the epoch's order, one claim
+// ahead, and the next rows' first entries are read while the current rows run.
+template <typename T, int NC, int G, int CH>
+__global__ void __launch_bounds__(ROW_BLOCK, ROW_BLOCKS)
+    sgd_rows_kernel(const RowTask* __restrict__ tasks, int32_t nrows, const int32_t* __restrict__ list,
+                    T* __restrict__ Y, int dim, int* __restrict__ counter, const StepParams<T> p) {
     const int lane = threadIdx.x & 31;
-    const float ef = p.epoch;
-    const int64_t j0 = r.ptr[h], r1 = r.ptr[h + 1];
-    int32_t nbase;
-    uint32_t nsize;
-    instance_range(h, p, nbase, nsize);
-    float hx = 0.0f, hy = 0.0f;   // lane 0: the head
-    bool have = false;
-    for (int64_t c = j0; c < r1; c += 32) {
-        float2 seen = make_float2(0.0f, 0.0f);
-        const bool resync = lane == 0 && have;
-        if (resync) seen = ld_relaxed_f2(&Y[h]);   // includes this lane's earlier publications
-        const float cx = hx, cy = hy;                          // lane 0: the head at the chunk's start
-        const int64_t j = c + lane;
-        bool fire = false;
-        if (j < r1) {
-            const float en = r.enext[j];
-            fire = en <= ef;
-            if (fire) {
-                const float ep = r.eps[j], enn = r.enneg[j];
-                const int32_t t = r.targets[j];
-                const float epns = ep / p.rate;
-                const int nn = static_cast<int>((ef - enn) / epns);
-                r.enext[j] = en + ep;
-                r.enneg[j] = enn + static_cast<float>(nn) * epns;
-                const int draws = nn > 0 ? nn : 0;
-                ++fired;
-                drawn += draws;
-                HubEvent<NB>& e = ev[lane];
-                e.t = t;
-                e.nn = draws;
-                e.yt = __ldcg(&Y[t]);
-                NegStream rng(static_cast<uint32_t>(h), static_cast<uint32_t>(t), p.epoch_u, p.k0, p.k1);
-                const int m = draws < NB ? draws : NB;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    if (b < m) {
-                        const int32_t k = nbase + rng.bounded(nsize);
-                        e.ks[b] = k;
-                        e.yk[b] = __ldcg(&Y[k]);
-                    }
-                }
-            }
-        }
-        unsigned mask = __ballot_sync(0xffffffffu, fire);
-        __syncwarp();
-        if (lane == 0) {
-            if (mask && !have) {
-                const float2 y0 = ld_relaxed_f2(&Y[h]);
-                hx = y0.x;
-                hy = y0.y;
-                have = true;
-            }
-            while (mask) {
-                const int q = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const HubEvent<NB>& e = ev[q];
-                const float sx = hx, sy = hy;
-                {
-                    const float dx = hx - e.yt.x, dy = hy - e.yt.y;
-                    const float d2 = floor_eps(__fmaf_rn(dx, dx, dy * dy));
-                    const float cf = attract_coef_fast(d2, p);
-                    const float gx = p.alpha * clamp4(cf * dx);
-                    const float gy = p.alpha * clamp4(cf * dy);
-                    hx += gx;
-                    hy += gy;
-                    atomicAdd(&Y[e.t], make_float2(-gx, -gy));
-                }
-                const int nn = e.nn;
-                const int m = nn < NB ? nn : NB;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    if (b < m && e.ks[b] != h) {
-                        const float dx = hx - e.yk[b].x, dy = hy - e.yk[b].y;
-                        const float d2 = floor_eps(__fmaf_rn(dx, dx, dy * dy));
-                        const float cf = repulse_coef_fast(d2, p);
-                        hx = __fmaf_rn(p.alpha, clamp4(cf * dx), hx);
-                        hy = __fmaf_rn(p.alpha, clamp4(cf * dy), hy);
-                    }
-                }
-                if (nn > NB) {   // rare: the rest of this edge's negative samples, from the same stream
-                    NegStream rng(static_cast<uint32_t>(h), static_cast<uint32_t>(e.t), p.epoch_u, p.k0, p.k1);
-                    for (int b = 0; b < nn; ++b) {
-                        const int32_t k = nbase + rng.bounded(nsize);
-                        if (b < NB || k == h) continue;
-                        const float2 y = __ldcg(&Y[k]);
-                        const float dx = hx - y.x, dy = hy - y.y;
-                        const float d2 = floor_eps(__fmaf_rn(dx, dx, dy * dy));
-                        const float cf = repulse_coef_fast(d2, p);
-                        hx = __fmaf_rn(p.alpha, clamp4(cf * dx), hx);
-                        hy = __fmaf_rn(p.alpha, clamp4(cf * dy), hy);
-                    }
-                }
-                atomicAdd(&Y[h], make_float2(hx - sx, hy - sy));
-            }
-            if (resync) {   // a read was issued at this chunk's start
-                hx = seen.x + (hx - cx);
-                hy = seen.y + (hy - cy);
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// The epoch: warps first take the hub rows, one per warp, from counter[0];
-// then the other rows 32 at a time from counter[1], one per lane, each loop
-// iteration applying one firing edge of every lane's row (the rows a warp
-// takes have similar lengths: row_order_key_kernel, and per epoch
-// epoch_bulk_order_kernel).
-template <int NB, int MINB, bool FRESH>
-__global__ void __launch_bounds__(256, MINB) sgd_rows_2d_f32(RowArgs<float> r, float2* __restrict__ Y,
-                                                             SgdParams<float> p) {
-    __shared__ HubEvent<NB> hub_ev[256 / 32][32];
-    __shared__ float scan_win[256 / 32][2 * BULK_CHUNK * 32];
-    unsigned long long fired = 0, drawn = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    while (true) {
-        int32_t u = 0;
-        if (lane == 0) u = atomicAdd(&r.counter[0], 1);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if (u >= r.nhub) break;
-        hub_row<NB>(r.order[u], r, Y, p, hub_ev[warp], fired, drawn);
-        __syncwarp();
-    }
-    const int32_t nbulk = r.nrows - r.nhub;
-    const int32_t* bulk = r.bulk ? r.bulk : r.order + r.nhub;
-    while (true) {
+    auto claim = [&](RowTask& r) {   // false: none left
         int32_t base = 0;
-        if (lane == 0) base = atomicAdd(&r.counter[1], 32);
+        if (lane == 0) base = atomicAdd(counter, 32 / G);
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= nbulk) break;
-        LaneRow L;
-        L.h = -1;
-        const int32_t idx = base + lane;
-        if (idx < nbulk && !lane_row_start(L, bulk[idx], r, Y, p, &scan_win[warp][lane])) L.h = -1;
-        while (__any_sync(0xffffffffu, L.h >= 0)) {
-            if (L.h >= 0 && !lane_row_step<NB, FRESH>(L, r, Y, p, fired, drawn)) L.h = -1;
+        const int32_t i = base + lane / G;
+        r = RowTask{0, 0, 0, 0};
+        if (i < nrows) {
+            const int4 q = __ldg(reinterpret_cast<const int4*>(tasks) + i);
+            r = RowTask{q.x, static_cast<uint32_t>(q.y), static_cast<uint32_t>(q.z), 0};
         }
-    }
-    add_totals(r.totals, fired, drawn);
-}
-
-struct Sgd2dVariant {
-    void (*kernel)(RowArgs<float>, float2*, SgdParams<float>);
-    int neg_batch, min_blocks;
-};
-const Sgd2dVariant SGD_2D_VARIANTS[] = {
-    // default: head kept in registers, published per firing edge, negative
-    // samples gathered 5 at a time (most firing edges draw 5; measured at
-    // 1M: 180 ms against 185 for 6, 186 for 4, 189 for 8)
-    {sgd_rows_2d_f32<5, 2, false>, 5, 2},
-    {sgd_rows_2d_f32<6, 2, false>, 6, 2},
-    {sgd_rows_2d_f32<6, 3, false>, 6, 3},
-    {sgd_rows_2d_f32<8, 2, false>, 8, 2},
-    {sgd_rows_2d_f32<6, 2, true>, 6, 2},     // head re-read before every firing edge
-    {sgd_rows_2d_f32<4, 2, false>, 4, 2},
-};
-constexpr int NUM_SGD_2D_VARIANTS = sizeof(SGD_2D_VARIANTS) / sizeof(SGD_2D_VARIANTS[0]);
-
-// Any dimension (up to MAX_GENERIC_DIM) and either precision; same per-row order.
-template <typename T>
-__global__ void __launch_bounds__(128) sgd_rows_generic(RowArgs<T> r, T* __restrict__ Y, int dim, SgdParams<T> p) {
-    T head[MAX_GENERIC_DIM], pub[MAX_GENERIC_DIM];
-    unsigned long long fired = 0, drawn = 0;
-    const T ef = p.epoch;
+        return base < nrows;
+    };
+    RowTask cur, nxt;
+    if (!claim(cur)) return;
+    ListHead<CH> head_of_list;
+    head_of_list.load(list, cur.start8, cur.count);
     while (true) {
-        const int32_t base = claim_rows(r.counter);
-        if (base >= r.nrows) break;
-        const int32_t i = base + (threadIdx.x & 31);
-        if (i < r.nrows) {
-            const int32_t h = r.order[i];
-            const int64_t r1 = r.ptr[h + 1];
-            int64_t j = next_firing(r.enext, r.ptr[h], r1, ef);
-            if (j < r1) {
-                int32_t nbase;
-                uint32_t nsize;
-                instance_range(h, p, nbase, nsize);
-                T* yh = Y + static_cast<size_t>(h) * dim;
-                for (int d = 0; d < dim; ++d) head[d] = pub[d] = __ldcg(yh + d);
-                int since = 0;
-                do {
-                    const T ep = r.eps[j];
-                    const T epns = ep / p.rate;
-                    const T enn = r.enneg[j];
-                    const int nn = static_cast<int>((ef - enn) / epns);
-                    r.enext[j] = r.enext[j] + ep;
-                    r.enneg[j] = enn + static_cast<T>(nn) * epns;
-                    const int32_t t = r.targets[j];
-                    ++fired;
-                    drawn += nn > 0 ? nn : 0;
-                    T* yt = Y + static_cast<size_t>(t) * dim;
-                    T d2 = 0;
-                    for (int d = 0; d < dim; ++d) {
-                        const T diff = head[d] - __ldcg(yt + d);
-                        d2 += diff * diff;
-                    }
-                    {
-                        const T c = attract_coef(floor_eps(d2), p);
-                        for (int d = 0; d < dim; ++d) {
-                            const T g = p.alpha * clamp4(c * (head[d] - __ldcg(yt + d)));
-                            head[d] += g;
-                            atomicAdd(yt + d, -g);
-                        }
-                    }
-                    if (nn > 0) {
-                        NegStream rng(static_cast<uint32_t>(h), static_cast<uint32_t>(t), p.epoch_u, p.k0, p.k1);
-                        for (int q = 0; q < nn; ++q) {
-                            const int32_t k = nbase + rng.bounded(nsize);
-                            if (k == h) continue;
-                            const T* yk = Y + static_cast<size_t>(k) * dim;
-                            T dd2 = 0;
-                            for (int d = 0; d < dim; ++d) {
-                                const T diff = head[d] - __ldcg(yk + d);
-                                dd2 += diff * diff;
-                            }
-                            const T c = repulse_coef(floor_eps(dd2), p);
-                            for (int d = 0; d < dim; ++d) head[d] += p.alpha * clamp4(c * (head[d] - __ldcg(yk + d)));
-                        }
-                    }
-                    j = next_firing(r.enext, j + 1, r1, ef);
-                    if (++since >= p.publish_every || j >= r1) {
-                        for (int d = 0; d < dim; ++d) {
-                            atomicAdd(yh + d, head[d] - pub[d]);
-                            pub[d] = head[d];
-                        }
-                        since = 0;
-                    }
-                } while (j < r1);
-            }
-        }
+        const bool more = claim(nxt);
+        Point<T, NC, G> head;
+        head.load(Y, cur.row, dim);
+        walk_row<T, NC, G, CH, false>(head, cur.row, head_of_list, Y, dim, p);
         __syncwarp();
+        if (!more) break;
+        cur = nxt;
+        head_of_list.load(list, cur.start8, cur.count);
     }
-    add_totals(r.totals, fired, drawn);
 }
 
 // ------------------------------------------------------------ transform --
@@ -823,12 +536,12 @@ __global__ void __launch_bounds__(128) sgd_rows_generic(RowArgs<T> r, T* __restr
 // applied to points added to a finished layout).  Row i of the transform
 // graph holds new point i's nearest reference points with their smoothed
 // similarities; it is optimised like a row of optimize_layout
-// (optimize_layout.hpp:136-180: schedule, attractive step, negative samples,
-// the same arithmetic as sgd_rows_generic) except that only the new point
-// moves: the reference points it is pulled to and the negative samples,
-// drawn among the reference points, stay fixed.  Rows then share nothing that
-// changes, so one thread takes one row through all epochs in one launch and
-// the result does not depend on the launch shape.
+// (optimize_layout.hpp:136-180: schedule, attractive step, negative samples)
+// except that only the new point moves: the reference points it is pulled to
+// and the negative samples, drawn among the reference points, stay fixed.
+// Rows then share nothing that changes, so one thread (or lane group) takes
+// one row through all epochs of a window in one launch and the result does
+// not depend on the launch shape.
 
 // Initial position of every new point: the mean of its neighbours' reference
 // positions weighted by the similarities (FP64 sums in edge order; plain mean
@@ -854,70 +567,72 @@ __global__ void transform_init_kernel(int32_t nq, int dim, const int64_t* __rest
     }
 }
 
-// All epochs of every new point's row (thread i: row i).  head0 + i is the
-// point's index in the negative-sample stream's counter; lr is the learning
-// rate in the layout's type.
-template <typename T>
-__global__ void __launch_bounds__(128)
-    transform_sgd_kernel(int32_t nq, int dim, const int64_t* __restrict__ ptr, const int32_t* __restrict__ targets,
-                         const T* __restrict__ eps, T* __restrict__ enext, T* __restrict__ enneg,
-                         const T* __restrict__ Yref, int32_t nref, T* __restrict__ Ynew, int32_t head0, int num_epochs,
-                         T lr, SgdParams<T> p) {
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq) return;
-    T head[MAX_GENERIC_DIM];
-    T* yh = Ynew + static_cast<size_t>(i) * dim;
-    for (int d = 0; d < dim; ++d) head[d] = yh[d];
-    const int64_t r0 = ptr[i], r1 = ptr[i + 1];
-    const uint32_t hid = static_cast<uint32_t>(head0 + i);
-    for (int e = 0; e < num_epochs; ++e) {
-        const T ef = static_cast<T>(e);
+// The epochs [first, first + epochs) of every new point's row (lane group i: row i).
+template <typename T, int NC, int G, int CH>
+__global__ void __launch_bounds__(ROW_BLOCK, ROW_BLOCKS)
+    transform_rows_kernel(int32_t nq, const ListSpan* __restrict__ span, const int32_t* __restrict__ list,
+                          const T* __restrict__ Yref, T* __restrict__ Ynew, int dim, int first, int epochs, int total,
+                          T lr, StepParams<T> p) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * ROW_BLOCK + threadIdx.x) / G;
+    const int32_t row = i < nq ? static_cast<int32_t>(i) : 0;
+    Point<T, NC, G> head;
+    head.load(Ynew, row, dim);
+    for (int e = 0; e < epochs; ++e) {
+        const T ef = static_cast<T>(first + e);
         // alpha as in the layout's epochs (optimize_layout.hpp:132-133)
-        const T alpha = static_cast<T>(static_cast<double>(lr) *
-                                       (1.0 - static_cast<double>(ef / static_cast<T>(num_epochs))));
-        for (int64_t j = r0; j < r1; ++j) {
-            if (!(enext[j] <= ef)) continue;
-            const T ep = eps[j];
-            const T epns = ep / p.rate;
-            const T enn = enneg[j];
-            const int nn = static_cast<int>((ef - enn) / epns);
-            enext[j] = enext[j] + ep;
-            enneg[j] = enn + static_cast<T>(nn) * epns;
-            const int32_t t = targets[j];
-            const T* yt = Yref + static_cast<size_t>(t) * dim;
-            T d2 = 0;
-            for (int d = 0; d < dim; ++d) {
-                const T diff = head[d] - yt[d];
-                d2 += diff * diff;
-            }
-            {
-                const T c = attract_coef(floor_eps(d2), p);
-                for (int d = 0; d < dim; ++d) head[d] += alpha * clamp4(c * (head[d] - yt[d]));
-            }
-            if (nn > 0) {
-                NegStream rng(hid, static_cast<uint32_t>(t), static_cast<uint32_t>(e), p.k0, p.k1);
-                for (int q = 0; q < nn; ++q) {
-                    const T* yk = Yref + static_cast<size_t>(rng.bounded(static_cast<uint32_t>(nref))) * dim;
-                    T dd2 = 0;
-                    for (int d = 0; d < dim; ++d) {
-                        const T diff = head[d] - yk[d];
-                        dd2 += diff * diff;
-                    }
-                    const T c = repulse_coef(floor_eps(dd2), p);
-                    for (int d = 0; d < dim; ++d) head[d] += alpha * clamp4(c * (head[d] - yk[d]));
-                }
-            }
-        }
+        p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(ef / static_cast<T>(total))));
+        const ListSpan sp = span[static_cast<int64_t>(e) * nq + row];
+        ListHead<CH> l;
+        l.load(list, sp.start8, i < nq ? sp.end - sp.start8 * LIST_ALIGN : 0u);
+        walk_row<T, NC, G, CH, true>(head, row, l, const_cast<T*>(Yref), dim, p);
     }
-    for (int d = 0; d < dim; ++d) yh[d] = head[d];
+    if (i < nq) head.each(Ynew, row, dim, [](T& x, const T* q) { *const_cast<T*>(q) = x; });
 }
 
-// UMAPB_CHECK_SCHEDULE=1: the epoch kernels count the firing edges and
-// negative samples they process, and every run compares the counts with the
+// out, rows of 'to' coordinates, from in, rows of 'from' (the missing ones 0).
+template <typename T>
+__global__ void restride_kernel(size_t values, const T* __restrict__ in, int from, T* __restrict__ out, int to) {
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < values; i += size_t(gridDim.x) * blockDim.x) {
+        const size_t row = i / to;
+        const int c = static_cast<int>(i % to);
+        out[i] = c < from ? in[row * from + c] : T(0);
+    }
+}
+
+// Calls f with the coordinates per lane, lanes per row and entries in flight
+// for a layout of 'dim' dimensions: one thread per row while the points in
+// flight fit its registers, else the smallest group of lanes.
+template <typename T, class F>
+void for_dim(int dim, F f) {
+    using std::integral_constant;
+    auto go = [&](auto nc, auto g, auto ch) { f(nc, g, ch); };
+    // gathers in flight per lane cover an L2 access: 8 float steps, 4 double ones
+    constexpr int deep = sizeof(T) == 4 ? 8 : 4;
+#define UMAPB_SHAPE(NC, G, CH) go(integral_constant<int, NC>(), integral_constant<int, G>(), integral_constant<int, CH>())
+    if (dim == 1) UMAPB_SHAPE(1, 1, deep);
+    else if (dim == 2) UMAPB_SHAPE(2, 1, deep);
+    else if (dim == 4) UMAPB_SHAPE(4, 1, deep);
+    else if (dim <= 8) UMAPB_SHAPE(1, 8, deep);
+    else if (dim <= 16) UMAPB_SHAPE(1, 16, deep);
+    else if (dim <= 32) UMAPB_SHAPE(1, 32, deep);
+    else UMAPB_SHAPE(2, 32, deep);
+#undef UMAPB_SHAPE
+}
+
+// UMAPB_CHECK_SCHEDULE=1: the lists' firing edges and negative samples are
+// counted as they are written, and every run compares the counts with the
 // schedule's own totals (sched_totals_kernel).
 bool check_schedule() {
     const char* e = std::getenv("UMAPB_CHECK_SCHEDULE");
     return e && *e && *e != '0';
+}
+
+// Bytes of interaction lists held at once: at a million points ten epochs (the
+// schedule state is read and written once a window: 126 ms a run with 2 GB, 135
+// with 1 GB, 124 with 4 GB).  UMAPB_SGD_WINDOW_BYTES overrides it.
+size_t window_bytes() {
+    const char* e = std::getenv("UMAPB_SGD_WINDOW_BYTES");
+    return e && *e ? static_cast<size_t>(std::max(1ll, std::atoll(e))) : size_t(1) << 31;
 }
 
 int sm_count() {
@@ -931,33 +646,65 @@ int sm_count() {
     return count;
 }
 
-// Resident blocks per SM of 2-d variant v at 'block' threads (occupancy query, cached).
-int sgd_2d_resident(int v, int block) {
-    static int cache[NUM_SGD_2D_VARIANTS][2] = {};
-    const int bi = block == 128 ? 0 : 1;
-    if (cache[v][bi] == 0) {
-        int r = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, SGD_2D_VARIANTS[v].kernel, block, 0) != cudaSuccess || r < 1) {
-            cudaGetLastError();
-            r = 1;
-        }
-        cache[v][bi] = r;
-    }
-    return cache[v][bi];
+// Rows in flight at once: at most n / window_div (a sliding window over the
+// claim order), so that few rows run beside their neighbours with positions
+// read before those neighbours' updates, in steps of 256; small layouts take
+// min(n / 8, 32768).  At most 256 per SM: with eight gathers in flight each
+// they keep the SM's gather rate (one point per cycle) busy, and more leave
+// the longest rows a smaller share of it: a million points, 200 epochs take
+// 131 ms with 256, 148 with 512, 139 with 192.
+int64_t rows_in_flight(int32_t n, int window_div) {
+    const int64_t most = int64_t(ROW_BLOCK * ROW_BLOCKS) * sm_count();
+    if (window_div <= 0) return most;
+    const int64_t w = std::max<int64_t>(1, std::max<int64_t>(n / window_div, std::min<int64_t>(n / 8, 32768)));
+    return std::min(most, (w + 255) / 256 * 256);
 }
 
-int generic_resident() {
-    static int r = 0;
-    if (r == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, sgd_rows_generic<double>, 128, 0) != cudaSuccess || r < 1) {
+// Blocks of the epoch kernel that are resident at once on the device.
+template <typename T, int NC, int G, int CH>
+int64_t resident_blocks() {
+    static int per_sm = 0;
+    if (per_sm == 0) {
+        int r = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, sgd_rows_kernel<T, NC, G, CH>, ROW_BLOCK, 0) != cudaSuccess ||
+            r < 1) {
             cudaGetLastError();
             r = 1;
         }
+        per_sm = r;
     }
-    return r;
+    return static_cast<int64_t>(per_sm) * sm_count();
+}
+
+template <typename T>
+StepParams<T> step_params(double a, double b, double gamma) {
+    StepParams<T> p{};
+    p.a = static_cast<T>(a);
+    p.b = static_cast<T>(b);
+    p.neg2ab = T(-2) * p.a * p.b;
+    p.gamma2b = T(2) * static_cast<T>(gamma) * p.b;
+    return p;
+}
+
+ListStream list_stream(uint64_t seed, int32_t n) {
+    ListStream st;
+    st.k0 = static_cast<uint32_t>(seed) ^ RNG_NEGATIVE;
+    st.k1 = static_cast<uint32_t>(seed >> 32);
+    st.n = n;
+    return st;
 }
 
 }  // namespace
+
+template <typename T>
+SgdEngine<T>::~SgdEngine() {
+    for (cudaStream_t st : {epochs_stream_, lists_stream_}) {
+        if (st) {
+            cudaStreamSynchronize(st);
+            stream_put(st);
+        }
+    }
+}
 
 template <typename T>
 void SgdEngine<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s, int base_epoch) {
@@ -972,19 +719,19 @@ void SgdEngine<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s, int base_epo
         UMAPB_CUDA(cudaMemcpyAsync(enneg_.get(), ep->enneg0.get(), nnz * sizeof(T), cudaMemcpyDeviceToDevice, s));
     }
     state_epoch_ = base_epoch_;
-    // rows by descending firing rate
     order_.allocate(n, s);
     if (n > 0) {
         DevArray<uint64_t> key(n, s), key_sorted(n, s);
         DevArray<int32_t> row(n, s);
-        DevArray<int> cnt(1, s);
-        cnt.zero(s);
-        float hub_rate = static_cast<float>(HUB_RATE);   // UMAPB_SGD_HUB_RATE overrides it
-        if (const char* e = std::getenv("UMAPB_SGD_HUB_RATE")) hub_rate = static_cast<float>(std::atof(e));
+        DevArray<float> rate(n, s);
+        DevArray<unsigned long long> total(1, s);
+        total.zero(s);
         int32_t group = ORDER_GROUP;                       // UMAPB_SGD_ORDER_GROUP overrides it
         if (const char* e = std::getenv("UMAPB_SGD_ORDER_GROUP")) group = std::max(1, std::atoi(e));
-        row_order_key_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(n, ep->ptr.get(), ep->eps.get(), hub_rate, group,
-                                                                key.get(), row.get(), cnt.get());
+        row_rate_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(n, ep->ptr.get(), ep->eps.get(), rate.get(), total.get());
+        UMAPB_LAUNCH_CHECK();
+        row_order_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, rate.get(), total.get(), rows_in_flight(n, window_div),
+                                                              group, key.get(), row.get());
         UMAPB_LAUNCH_CHECK();
         int end_bit = 33;
         while (end_bit < 64 && (int64_t(1) << (end_bit - 32)) <= int64_t(n) / group + 1) ++end_bit;
@@ -994,11 +741,8 @@ void SgdEngine<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s, int base_epo
         DevArray<unsigned char> temp(tb, s);
         UMAPB_CUDA(cub::DeviceRadixSort::SortPairs(temp.get(), tb, key.get(), key_sorted.get(), row.get(), order_.get(),
                                                    n, 0, end_bit, s));
-        UMAPB_CUDA(cudaMemcpyAsync(&nhub_, cnt.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-        UMAPB_SYNC(s);
-    } else {
-        nhub_ = 0;
     }
+    lists_.setup(ep, s);
 }
 
 template <typename T>
@@ -1016,176 +760,103 @@ void SgdEngine<T>::state_at(int epoch, T* enext, T* enneg, cudaStream_t s) {
     }
 }
 
-// Autotuner: times one epoch with each candidate launch shape on scratch
-// copies of the layout and of the schedule state, keeps the fastest, and
-// remembers it per size class (log2 of the edge count).
-template <typename T>
-template <class Launch>
-void SgdEngine<T>::tune(T* Y, int num_dim, int epoch, Launch& launch, cudaStream_t s) {
-    static std::mutex mu;
-    static std::map<int, std::pair<int, int>> cache;   // size class -> (block, variant)
-    const int64_t nnz = ep_->nnz;
-    int key = 0;
-    while ((int64_t(1) << key) < nnz) ++key;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) {
-            block_ = it->second.first;
-            variant_ = it->second.second;
-            return;
-        }
-    }
-    const size_t total = static_cast<size_t>(ep_->n) * num_dim;
-    DevArray<T> yscr(total, s), en(nnz, s), enn(nnz, s);
-    DevArray<int> counter(2, s);
-    cudaEvent_t a = event_get(), b = event_get();
-    float best = 1e30f;
-    for (int v = 0; v < NUM_SGD_2D_VARIANTS; ++v) {
-        for (int blk : {128, 256}) {
-            UMAPB_CUDA(cudaMemcpyAsync(yscr.get(), Y, total * sizeof(T), cudaMemcpyDeviceToDevice, s));
-            UMAPB_CUDA(cudaMemcpyAsync(en.get(), enext_.get(), nnz * sizeof(T), cudaMemcpyDeviceToDevice, s));
-            UMAPB_CUDA(cudaMemcpyAsync(enn.get(), enneg_.get(), nnz * sizeof(T), cudaMemcpyDeviceToDevice, s));
-            counter.zero(s);
-            UMAPB_CUDA(cudaEventRecord(a, s));
-            launch(yscr.get(), en.get(), enn.get(), counter.get(), nullptr, epoch, blk, v);
-            UMAPB_CUDA(cudaEventRecord(b, s));
-            UMAPB_CUDA(cudaEventSynchronize(b));
-            float t = 0;
-            UMAPB_CUDA(cudaEventElapsedTime(&t, a, b));
-            if (t < best) {
-                best = t;
-                block_ = blk;
-                variant_ = v;
-            }
-        }
-    }
-    event_put(a);
-    event_put(b);
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = std::make_pair(block_, variant_);
-}
-
 template <typename T>
 void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double b, double gamma, double learning_rate,
-                       uint64_t seed, cudaStream_t caller, float* ms_schedule, float* ms_sgd) {
+                       uint64_t seed, cudaStream_t s, float* ms_schedule, float* ms_sgd) {
     if (ms_schedule) *ms_schedule = 0;
     if (ms_sgd) *ms_sgd = 0;
     if (last <= first) return;
-    require(num_dim >= 1 && num_dim <= MAX_GENERIC_DIM, "num_dim must be between 1 and 64");
+    require(num_dim >= 1 && num_dim <= MAX_DIM, "num_dim must be between 1 and 64");
     const int total = ep_->total_epochs;
-    SgdParams<T> p;
-    p.a = static_cast<T>(a);
-    p.b = static_cast<T>(b);
-    p.neg2ab = T(-2) * p.a * p.b;
-    p.gamma2b = T(2) * static_cast<T>(gamma) * p.b;
-    p.rate = ep_->negative_sample_rate;
-    p.k0 = static_cast<uint32_t>(seed) ^ RNG_NEGATIVE;
-    p.k1 = static_cast<uint32_t>(seed >> 32);
-    p.n = ep_->n;
-    p.publish_every = std::max(1, publish_every);
-    p.inst_start = inst_start_;
-    p.num_inst = num_inst_;
+    const int32_t n = ep_->n;
+    StepParams<T> p = step_params<T>(a, b, gamma);
+    ListStream stream = list_stream(seed, n);
+    stream.inst_start = inst_start_;
+    stream.num_inst = num_inst_;
     const T lr = static_cast<T>(learning_rate);
-    const bool use_2d = std::is_same<T, float>::value && num_dim == 2;
     const bool check = check_schedule();
-    cudaStream_t s = caller;
-    // Rows in flight at once: at most n / window_div (a sliding window over
-    // the claim order), so that few rows run beside their neighbours with
-    // positions read before those neighbours' updates; at a million points
-    // that is still enough rows to keep L2 saturated.
-    // UMAPB_SGD_MAX_BLOCKS overrides the block count (0: from the window).
-    int max_blocks = 0;
-    if (const char* e = std::getenv("UMAPB_SGD_MAX_BLOCKS")) max_blocks = std::max(0, std::atoi(e));
-    const int64_t window_rows = window_div > 0
-        ? std::max<int64_t>(1, std::max<int64_t>(ep_->n / window_div, std::min<int64_t>(ep_->n / 8, 32768)))
-        : int64_t(1) << 40;
-
-    const bool eorder = use_2d && epoch_order && ep_->n > nhub_;
-    if (eorder) {
-        next_count_.reserve(ep_->n, s);
-        bulk_.reserve(ep_->n - nhub_, s);
-    }
-    // One epoch launch on (Yp, schedule state en/enn), claiming rows from 'counter'.
-    auto launch = [&](T* Yp, T* en, T* enn, int* counter, unsigned long long* totals, int e_abs, int block,
-                      int variant) {
-        const T epoch_t = static_cast<T>(e_abs);
-        // alpha = lr * (1 - epoch / num_epochs) in the reference's types (optimize_layout.hpp:132-133)
-        p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(epoch_t / static_cast<T>(total))));
-        p.epoch = epoch_t;
-        p.epoch_u = static_cast<uint32_t>(e_abs);
-        RowArgs<T> r;
-        r.order = order_.get();
-        r.nrows = ep_->n;
-        r.ptr = ep_->ptr.get();
-        r.targets = ep_->targets.get();
-        r.eps = ep_->eps.get();
-        r.enext = en;
-        r.enneg = enn;
-        r.counter = counter;
-        r.totals = totals;
-        r.nhub = use_2d ? nhub_ : 0;
-        r.bulk = nullptr;
-        r.next_count = nullptr;
-        if (eorder) {
-            r.next_count = next_count_.get();
-            if (e_abs > first) {   // counts from the previous epoch of this call
-                const int32_t nbulk = ep_->n - nhub_;
-                epoch_bulk_order_kernel<<<static_cast<unsigned>((nbulk + ORDER_GROUP - 1) / ORDER_GROUP),
-                                          EPOCH_ORDER_THREADS, 0, s>>>(order_.get() + nhub_, nbulk,
-                                                                      next_count_.get(), bulk_.get());
-                UMAPB_LAUNCH_CHECK();
-                r.bulk = bulk_.get();
-            }
-        }
-        if (use_2d) {
-            if constexpr (std::is_same<T, float>::value) {
-                int64_t g = static_cast<int64_t>(sm_count()) * sgd_2d_resident(variant, block);
-                g = std::min<int64_t>(g, std::max<int64_t>(1, (window_rows + block - 1) / block));
-                if (max_blocks > 0) g = std::min<int64_t>(g, max_blocks);
-                SGD_2D_VARIANTS[variant].kernel<<<static_cast<unsigned>(g), block, 0, s>>>(
-                    r, reinterpret_cast<float2*>(Yp), p);
-            }
-        } else {
-            int64_t g = static_cast<int64_t>(sm_count()) * generic_resident();
-            g = std::min<int64_t>(g, std::max<int64_t>(1, (window_rows + 127) / 128));
-            if (max_blocks > 0) g = std::min<int64_t>(g, max_blocks);
-            sgd_rows_generic<T><<<static_cast<unsigned>(g), 128, 0, s>>>(r, Yp, num_dim, p);
-        }
-        UMAPB_LAUNCH_CHECK();
+    const int64_t rows = rows_in_flight(n, window_div);
+    // Points are read and added to as vectors of up to 16 bytes: a layout of
+    // three dimensions, and an array that is not aligned to them, is worked on
+    // in a copy (three dimensions as four, the fourth 0: one access each
+    // instead of three).
+    const int stride = num_dim == 3 ? 4 : num_dim;
+    const size_t values = static_cast<size_t>(n) * stride;
+    const bool copied = stride != num_dim || reinterpret_cast<uintptr_t>(Y) % 16 != 0;
+    DevArray<T> copy(copied ? values : 0, s);
+    T* Yp = copied ? copy.get() : Y;
+    const int E = last - first;
+    DevArray<int> counters(E, s);
+    DevArray<unsigned long long> totals(check ? 2 * static_cast<size_t>(E) : 0, s);
+    // The lists of the next window are built on one stream while this one's
+    // epochs run on the other, which goes first where both want a place.  When
+    // the epochs fill the device the two take turns instead: the epochs'
+    // gathers and the lists' shuffles and shared memory go through the same
+    // queue of an SM, and at a million points both side by side take 1.1 ms an
+    // epoch against 0.65 ms one after the other.
+    const bool overlap = rows < int64_t(ROW_BLOCK * ROW_BLOCKS) * sm_count();
+    if (!epochs_stream_) epochs_stream_ = stream_get(true);
+    if (!lists_stream_) lists_stream_ = stream_get();
+    cudaStream_t es = epochs_stream_, ls = overlap ? lists_stream_ : epochs_stream_;
+    cudaEvent_t start = event_get(), finish = event_get(), ready = event_get(), done[2] = {event_get(), event_get()};
+    auto settle = [&] {
+        event_put(start);
+        event_put(finish);
+        event_put(ready);
+        event_put(done[0]);
+        event_put(done[1]);
     };
-
-    if (state_epoch_ != first) {
-        state_at(first, enext_.get(), enneg_.get(), s);
-        state_epoch_ = first;
-    }
-    if (autotune && use_2d) tune(Y, num_dim, first, launch, s);
-    const int W = last - first;
-    DevArray<int> counters(2 * static_cast<size_t>(W), s);
-    DevArray<unsigned long long> totals(check ? 2 * static_cast<size_t>(W) : 0, s);
-    cudaEvent_t start = event_get(), finish = event_get();
-    cudaGraphExec_t exec = nullptr;
     try {
         UMAPB_CUDA(cudaEventRecord(start, s));
-        auto enqueue = [&] {
-            UMAPB_CUDA(cudaMemsetAsync(counters.get(), 0, 2 * W * sizeof(int), s));
-            if (check) UMAPB_CUDA(cudaMemsetAsync(totals.get(), 0, 2 * W * sizeof(unsigned long long), s));
-            for (int e = first; e < last; ++e)
-                launch(Y, enext_.get(), enneg_.get(), counters.get() + 2 * (e - first),
-                       check ? totals.get() + 2 * (e - first) : nullptr, e, block_, variant_);
-        };
-        if (use_graphs) {
-            // the epochs of this call as one CUDA graph
-            cudaGraph_t graph = nullptr;
-            UMAPB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            enqueue();
-            UMAPB_CUDA(cudaStreamEndCapture(s, &graph));
-            const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (ie != cudaSuccess) cuda_fail(ie, "cudaGraphInstantiate", __FILE__, __LINE__);
-            UMAPB_CUDA(cudaGraphLaunch(exec, s));
-        } else {
-            enqueue();
+        if (state_epoch_ != first) state_at(first, enext_.get(), enneg_.get(), s);
+        state_epoch_ = -1;   // until the call has succeeded
+        counters.zero(s);
+        if (check) totals.zero(s);
+        if (copied && n > 0) {
+            restride_kernel<T><<<grid_for(values, 256), 256, 0, s>>>(values, Y, num_dim, Yp, stride);
+            UMAPB_LAUNCH_CHECK();
+        }
+        UMAPB_CUDA(cudaEventRecord(ready, s));
+        UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
+        UMAPB_CUDA(cudaStreamWaitEvent(ls, ready, 0));
+        const int window = lists_.window_epochs(overlap ? window_bytes() / 2 : window_bytes());
+        lists_.prepare(first, std::min(window, E), enext_.get(), enneg_.get(), overlap, ls);
+        int buffer = 0;
+        for (int e0 = first, windows = 0; e0 < last; ++windows) {
+            if (overlap) buffer = windows & 1;   // in turns one is enough
+            // the buffer's last epochs are done with it
+            if (overlap && windows >= 2) UMAPB_CUDA(cudaStreamWaitEvent(ls, done[buffer], 0));
+            const int W = lists_.build(buffer, enext_.get(), enneg_.get(), stream,
+                                       check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
+            if (n > 0) {
+                tasks_[buffer].reserve(static_cast<size_t>(W) * n, ls);
+                epoch_order_kernel<<<dim3((n - 1) / ORDER_GROUP + 1, W), EPOCH_ORDER_THREADS, 0, ls>>>(
+                    order_.get(), n, epoch_order, lists_.spans(buffer), tasks_[buffer].get());
+                UMAPB_LAUNCH_CHECK();
+            }
+            UMAPB_CUDA(cudaEventRecord(ready, ls));
+            UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
+            if (e0 + W < last) lists_.prepare(e0 + W, std::min(window, last - e0 - W), enext_.get(), enneg_.get(), overlap, ls);
+            for (int e = e0; e < e0 + W && n > 0; ++e) {
+                const T epoch_t = static_cast<T>(e);
+                // alpha = lr * (1 - epoch / num_epochs) in the reference's types (optimize_layout.hpp:132-133)
+                p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(epoch_t / static_cast<T>(total))));
+                for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
+                    constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
+                    const int64_t blocks = std::min((rows * G + ROW_BLOCK - 1) / ROW_BLOCK, resident_blocks<T, NC, G, CH>());
+                    sgd_rows_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), ROW_BLOCK, 0, es>>>(
+                        tasks_[buffer].get() + static_cast<size_t>(e - e0) * n, n, lists_.list(buffer), Yp, stride,
+                        counters.get() + (e - first), p);
+                });
+                UMAPB_LAUNCH_CHECK();
+            }
+            UMAPB_CUDA(cudaEventRecord(done[buffer], es));
+            e0 += W;
+        }
+        UMAPB_CUDA(cudaStreamWaitEvent(s, done[buffer], 0));   // the last window's: the lists came before it
+        if (copied && n > 0) {
+            restride_kernel<T><<<grid_for(values, 256), 256, 0, s>>>(static_cast<size_t>(n) * num_dim, Yp, stride, Y, num_dim);
+            UMAPB_LAUNCH_CHECK();
         }
         UMAPB_CUDA(cudaEventRecord(finish, s));
         UMAPB_CUDA(cudaEventSynchronize(finish));
@@ -1193,32 +864,23 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         UMAPB_CUDA(cudaEventElapsedTime(&ms, start, finish));
         if (ms_sgd) *ms_sgd = ms;
     } catch (...) {
-        // an error inside a graph capture leaves s capturing: end and drop it
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
-            cudaGraph_t g = nullptr;
-            cudaStreamEndCapture(s, &g);
-            if (g) cudaGraphDestroy(g);
-        }
         cudaGetLastError();
+        cudaStreamSynchronize(ls);   // nothing may still use what is released on the way out
+        cudaStreamSynchronize(es);
         cudaStreamSynchronize(s);
-        if (exec) cudaGraphExecDestroy(exec);
-        event_put(start);
-        event_put(finish);
+        settle();
         throw;
     }
-    if (exec) cudaGraphExecDestroy(exec);
-    event_put(start);
-    event_put(finish);
+    settle();
     state_epoch_ = last;
     if (check) {
-        std::vector<int64_t> want(2 * static_cast<size_t>(W));
+        std::vector<int64_t> want(2 * static_cast<size_t>(E));
         counts(first, last, want.data(), s);
-        std::vector<unsigned long long> got(2 * static_cast<size_t>(W));
+        std::vector<unsigned long long> got(2 * static_cast<size_t>(E));
         UMAPB_CUDA(cudaMemcpyAsync(got.data(), totals.get(), got.size() * sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, s));
         UMAPB_SYNC(s);
-        for (int w = 0; w < W; ++w)
+        for (int w = 0; w < E; ++w)
             require(static_cast<int64_t>(got[2 * w]) == want[2 * w] && static_cast<int64_t>(got[2 * w + 1]) == want[2 * w + 1],
                     "schedule self-check failed at epoch " + std::to_string(first + w), UMAPB_ERR_CUDA);
     }
@@ -1245,15 +907,6 @@ void SgdEngine<T>::counts(int first, int last, int64_t* out, cudaStream_t s) {
     for (size_t i = 0; i < h.size(); ++i) out[i] = static_cast<int64_t>(h[i]);
 }
 
-// UMAPB_SGD_VARIANT selects the 2-d kernel variant (index into
-// SGD_2D_VARIANTS) when the launch shape is not tuned.
-template <typename T>
-int SgdEngine<T>::default_variant() {
-    const char* e = std::getenv("UMAPB_SGD_VARIANT");
-    const int x = e ? std::atoi(e) : -1;
-    return (x >= 0 && x < NUM_SGD_2D_VARIANTS) ? x : 0;
-}
-
 // UMAPB_SGD_WINDOW_DIV: rows in flight at most max(n / this, min(n / 8, 32768))
 // (default 12; 0: no cap).
 template <typename T>
@@ -1270,15 +923,6 @@ bool SgdEngine<T>::default_epoch_order() {
     return !(e && std::atoi(e) == 0);
 }
 
-// UMAPB_SGD_PUBLISH_EVERY: firing edges between publications of a row's head
-// (default 1: after every firing edge).
-template <typename T>
-int SgdEngine<T>::default_publish_every() {
-    const char* e = std::getenv("UMAPB_SGD_PUBLISH_EVERY");
-    const int x = e ? std::atoi(e) : 0;
-    return (x >= 1 && x <= 1 << 20) ? x : 1;
-}
-
 template class SgdEngine<float>;
 template class SgdEngine<double>;
 
@@ -1293,31 +937,53 @@ void transform_init(int32_t nq, int num_dim, const int64_t* ptr, const int32_t* 
 template <typename T>
 void transform_layout(const DeviceEpochs<T>& ep, int num_dim, const T* Yref, int32_t nref, T* Ynew, int32_t head0,
                       double a, double b, double gamma, double learning_rate, uint64_t seed, cudaStream_t s) {
-    require(num_dim >= 1 && num_dim <= MAX_GENERIC_DIM, "num_dim must be between 1 and 64");
+    require(num_dim >= 1 && num_dim <= MAX_DIM, "num_dim must be between 1 and 64");
     require(nref >= 1, "the transform needs at least one reference point");
     const int32_t nq = ep.n;
     if (nq <= 0) return;
-    SgdParams<T> p{};
-    p.a = static_cast<T>(a);
-    p.b = static_cast<T>(b);
-    p.neg2ab = T(-2) * p.a * p.b;
-    p.gamma2b = T(2) * static_cast<T>(gamma) * p.b;
-    p.rate = ep.negative_sample_rate;
-    p.k0 = static_cast<uint32_t>(seed) ^ RNG_NEGATIVE;
-    p.k1 = static_cast<uint32_t>(seed >> 32);
-    p.n = nref;
-    p.publish_every = 1;
-    p.inst_start = nullptr;
-    p.num_inst = 1;
+    const StepParams<T> p = step_params<T>(a, b, gamma);
+    ListStream stream = list_stream(seed, nref);
+    stream.head0 = head0;
     DevArray<T> en(std::max<int64_t>(ep.nnz, 1), s), enn(std::max<int64_t>(ep.nnz, 1), s);
     if (ep.nnz) {
         UMAPB_CUDA(cudaMemcpyAsync(en.get(), ep.enext0.get(), ep.nnz * sizeof(T), cudaMemcpyDeviceToDevice, s));
         UMAPB_CUDA(cudaMemcpyAsync(enn.get(), ep.enneg0.get(), ep.nnz * sizeof(T), cudaMemcpyDeviceToDevice, s));
     }
-    transform_sgd_kernel<T><<<static_cast<unsigned>((nq + 127) / 128), 128, 0, s>>>(
-        nq, num_dim, ep.ptr.get(), ep.targets.get(), ep.eps.get(), en.get(), enn.get(), Yref, nref, Ynew, head0,
-        ep.total_epochs, static_cast<T>(learning_rate), p);
-    UMAPB_LAUNCH_CHECK();
+    // as in SgdEngine::run: vectors, so three dimensions and unaligned arrays go through copies
+    const int stride = num_dim == 3 ? 4 : num_dim;
+    DevArray<T> ref_copy, new_copy;
+    auto vectors = [&](const T* from, int32_t n, DevArray<T>& to) -> const T* {
+        if (stride == num_dim && reinterpret_cast<uintptr_t>(from) % 16 == 0) return from;
+        const size_t values = static_cast<size_t>(n) * stride;
+        to.allocate(values, s);
+        restride_kernel<T><<<grid_for(values, 256), 256, 0, s>>>(values, from, num_dim, to.get(), stride);
+        UMAPB_LAUNCH_CHECK();
+        return to.get();
+    };
+    Yref = vectors(Yref, nref, ref_copy);
+    T* Yp = const_cast<T*>(vectors(Ynew, nq, new_copy));
+    InteractionLists<T> lists;
+    lists.setup(&ep, s);
+    const int last = ep.total_epochs, window = lists.window_epochs(window_bytes());
+    lists.prepare(0, std::min(window, last), en.get(), enn.get(), false, s);
+    for (int e0 = 0; e0 < last;) {
+        const int W = lists.build(0, en.get(), enn.get(), stream, nullptr, false, s);
+        if (e0 + W < last) lists.prepare(e0 + W, std::min(window, last - e0 - W), en.get(), enn.get(), false, s);
+        for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
+            constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
+            const int64_t threads = static_cast<int64_t>(nq) * G;
+            transform_rows_kernel<T, NC, G, CH><<<static_cast<unsigned>((threads + ROW_BLOCK - 1) / ROW_BLOCK), ROW_BLOCK,
+                                                  0, s>>>(nq, lists.spans(0), lists.list(0), Yref, Yp, stride, e0, W, last,
+                                                          static_cast<T>(learning_rate), p);
+        });
+        UMAPB_LAUNCH_CHECK();
+        e0 += W;
+    }
+    if (Yp != Ynew) {
+        const size_t values = static_cast<size_t>(nq) * num_dim;
+        restride_kernel<T><<<grid_for(values, 256), 256, 0, s>>>(values, Yp, stride, Ynew, num_dim);
+        UMAPB_LAUNCH_CHECK();
+    }
 }
 
 template void transform_init<float>(int32_t, int, const int64_t*, const int32_t*, const float*, const float*, float*,

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "sgd_lists.cuh"
 
 namespace umapb {
 
@@ -179,11 +180,15 @@ template <typename T>
 void random_init(int32_t n, int num_dim, T* Y, uint64_t seed, double scale, cudaStream_t s);
 
 // ---- SGD (sgd.cu) -----------------------------------------------------------
-// Epochs of the reference's SGD: one thread per head row, the schedule
-// advanced in place in the reference's Float_ arithmetic (see sgd.cu).
+// Epochs of the reference's SGD: one thread or lane group per head row, over
+// lists built ahead in the reference's Float_ arithmetic (sgd_lists.cu, sgd.cu).
 template <typename T>
 class SgdEngine {
 public:
+    SgdEngine() = default;
+    SgdEngine(const SgdEngine&) = delete;
+    SgdEngine& operator=(const SgdEngine&) = delete;
+    ~SgdEngine();
     // ep->enext0 / enneg0 describe the schedule at epoch 'base_epoch'.
     void setup(const DeviceEpochs<T>* ep, cudaStream_t s, int base_epoch = 0);
     // Runs epochs [first, last) on Y (n x num_dim, device).  ms_schedule is
@@ -200,39 +205,24 @@ public:
         inst_start_ = inst_start;
         num_inst_ = num_inst;
     }
-    // Record the epochs of each run() call as one CUDA graph and launch that.
-    bool use_graphs = false;
-    // Pick the 2-d epoch kernel's block size and variant by timing the
-    // candidates on scratch copies (sgd.cu, tune()).
-    bool autotune = false;
-    // Firing edges between publications of a row's head (sgd.cu).
-    int publish_every = default_publish_every();
     // Rows in flight at most n / window_div (sgd.cu, run(); 0: no cap).
     int window_div = default_window_div();
-    // 2-d kernel: each epoch after the first of a run() call claims its rows
-    // sorted by this epoch's firing edges within chunks of the run's order
-    // (sgd.cu, epoch_bulk_order_kernel).
+    // Each epoch claims its rows sorted by their entries in this epoch within
+    // chunks of the run's order (sgd.cu, epoch_order_kernel).
     bool epoch_order = default_epoch_order();
-    int block_size() const { return block_; }
-    int variant() const { return variant_; }   // 2-d kernel variant (sgd.cu, SGD_2D_VARIANTS)
 
 private:
-    template <class Launch>
-    void tune(T* Y, int num_dim, int epoch, Launch& launch, cudaStream_t s);
-    static int default_variant();
-    static int default_publish_every();
     static int default_window_div();
     static bool default_epoch_order();
-    int block_ = 256, variant_ = default_variant();
     const DeviceEpochs<T>* ep_ = nullptr;
-    DevArray<uint16_t> next_count_;   // per row: firing edges in the next epoch
-    DevArray<int32_t> bulk_;          // this epoch's claim order of the non-hub rows
+    InteractionLists<T> lists_;
+    DevArray<RowTask> tasks_[2];      // per list buffer, [epoch of the window][position]: the rows in claim order
+    cudaStream_t epochs_stream_ = nullptr, lists_stream_ = nullptr;
     const int32_t* inst_start_ = nullptr;
     int32_t num_inst_ = 1;
     int base_epoch_ = 0;
     DevArray<T> enext_, enneg_;    // schedule state at state_epoch_
-    DevArray<int32_t> order_;      // rows by descending firing rate
-    int nhub_ = 0;                 // leading rows of order_ taken by a whole warp (2-d kernel)
+    DevArray<int32_t> order_;      // rows in the run's claim order
     int state_epoch_ = 0;          // epoch the state arrays describe
 };
 
