@@ -1,0 +1,58 @@
+"""Neighbour searches with more candidates than a thread's registers hold (the
+tensor-core search in several passes) and of queries against a reference set
+(its references split over several candidate lists), against the FP64 oracle:
+the same neighbours, except for exchanges of distances equal to 1e-6 relative,
+and distances rounded to float."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import same_neighbors
+
+pytestmark = pytest.mark.gpu
+
+
+def check(idx, dist, ridx, rdist):
+    assert same_neighbors(idx, ridx, rdist) == 0
+    np.testing.assert_allclose(dist.astype(np.float64), rdist, rtol=1e-6, atol=1e-30)
+
+
+@pytest.mark.parametrize("n,dim,k", [(700, 10, 25), (2900, 20, 40), (1500, 63, 56), (1300, 64, 57), (900, 127, 120),
+                                     (3000, 5, 88), (130, 3, 120), (400, 130, 40)])
+def test_knn_many_neighbours(umap, n, dim, k):
+    X = oracle.gaussian_mixture(n, dim, 4, 3.0, seed=n + k, dtype=np.float32)
+    check(*umap.knn(X, k), *oracle.knn(X, k))
+
+
+@pytest.mark.parametrize("k", [30, 70])
+def test_knn_many_neighbours_with_ties(umap, k):
+    # points of a small lattice: every distance many times, more equal ones than a pass lists
+    X = np.random.default_rng(5).integers(0, 4, size=(2000, 3)).astype(np.float32)
+    idx, dist = umap.knn(X, k)
+    ridx, rdist = oracle.knn(X, k)
+    np.testing.assert_allclose(dist.astype(np.float64), rdist, rtol=1e-6, atol=1e-30)
+    for row in idx:
+        assert len(set(row.tolist())) == k
+
+
+def test_knn_many_neighbours_without_scale(umap):
+    X = np.zeros((300, 6), np.float32)   # no finite non-zero maximum: the CUDA-core search
+    idx, dist = umap.knn(X, 40)
+    assert np.all(dist == 0) and np.all(idx >= 0)
+
+
+@pytest.mark.parametrize("nref,nq,dim,k", [(1023, 20, 8, 15), (1024, 130, 8, 15), (4096, 1, 8, 15), (5000, 129, 63, 15), (6000, 700, 64, 8), (5001, 300, 127, 24),
+                                           (4500, 260, 20, 30), (4200, 70, 30, 110), (4300, 40, 140, 15)])
+def test_query_against_references(umap, nref, nq, dim, k):
+    X = oracle.gaussian_mixture(nref + nq, dim, 5, 4.0, seed=nref + k, dtype=np.float32)
+    ref, new = X[:nref], np.vstack([X[nref:], X[:2]])   # the last two coincide with references
+    idx, dist = umap.knn_query(ref, new, k)
+    check(idx, dist, *oracle.knn_query(ref, new, k))
+    assert np.all(idx[-2:, 0] == np.arange(2)) and np.all(dist[-2:, 0] == 0)
+
+
+def test_query_far_from_references(umap):
+    # the queries set the scale of the search: the references' distances lose bits and are searched again in FP64
+    X = oracle.gaussian_mixture(4400, 12, 4, 3.0, seed=9, dtype=np.float32)
+    new = X[4100:] + np.float32(3000.0)
+    check(*umap.knn_query(X[:4100], new, 10), *oracle.knn_query(X[:4100], new, 10))

@@ -162,89 +162,162 @@ __global__ void __launch_bounds__(KNN_BLOCK) knn_bruteforce_kernel(const T* __re
     }
 }
 
+// Sorts 32 PER (distance, index) pairs held by a warp, pair e = 32 i + lane,
+// ascending: a bitonic network, partners in the same lane or a shuffle away.
+template <int PER>
+__device__ __forceinline__ void warp_sort(double (&d)[PER], int (&id)[PER]) {
+    const int lane = threadIdx.x & 31;
+    auto less = [](double x, int xi, double y, int yi) {   // index -1 (no candidate) maps above every index
+        return x < y || (x == y && static_cast<uint32_t>(xi) < static_cast<uint32_t>(yi));
+    };
+#pragma unroll
+    for (int size = 2; size <= 32 * PER; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= 32) {
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    const int o = i ^ (stride >> 5);
+                    if (o > i) {
+                        const bool up = ((32 * i + lane) & size) == 0;
+                        if (less(d[o], id[o], d[i], id[i]) == up) {
+                            const double x = d[i];
+                            d[i] = d[o];
+                            d[o] = x;
+                            const int y = id[i];
+                            id[i] = id[o];
+                            id[o] = y;
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    const double x = __shfl_xor_sync(0xffffffffu, d[i], stride);
+                    const int y = __shfl_xor_sync(0xffffffffu, id[i], stride);
+                    // the lower lane keeps the smaller of an ascending pair
+                    const bool small = (((32 * i + lane) & size) == 0) == ((lane & stride) == 0);
+                    if (small ? less(x, y, d[i], id[i]) : less(d[i], id[i], x, y)) {
+                        d[i] = x;
+                        id[i] = y;
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Squared distance of two rows, FP64, summed in coordinate order.
+__device__ __forceinline__ double distance2(const float* __restrict__ x, const float* __restrict__ y, int32_t dim,
+                                            bool vec4) {
+    double s = 0;
+    auto add = [&s](float u, float v) {
+        const double diff = static_cast<double>(u) - static_cast<double>(v);
+        s = __dadd_rn(s, __dmul_rn(diff, diff));
+    };
+    if (vec4) {   // rows of whole 16-byte vectors
+#pragma unroll 4
+        for (int d = 0; d < dim; d += 4) {
+            const float4 u = __ldg(reinterpret_cast<const float4*>(x + d)), v = __ldg(reinterpret_cast<const float4*>(y + d));
+            add(u.x, v.x);
+            add(u.y, v.y);
+            add(u.z, v.z);
+            add(u.w, v.w);
+        }
+    } else {
+#pragma unroll 4
+        for (int d = 0; d < dim; ++d) add(__ldg(x + d), __ldg(y + d));
+    }
+    return s;
+}
+
 // FP64 rescoring of the FP32 candidates of every query: keeps the best k by
 // (FP64 distance, index) and flags queries whose candidate set may miss a
-// true neighbour.
-template <int KCAP>
-__global__ void knn_rescore_kernel(const float* __restrict__ data, int32_t others, int32_t dim, int32_t k,
-                                   const int32_t* __restrict__ queries, int32_t nq, int cand_by_slot, int out_by_slot,
-                                   const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_d2,
-                                   int32_t* __restrict__ out_idx, float* __restrict__ out_dist,
-                                   double* __restrict__ out_dist64, int32_t* __restrict__ redo,
-                                   int32_t* __restrict__ redo_count, const float* __restrict__ norms,
-                                   const unsigned int* __restrict__ norm_max_bits, double tc_rel,
-                                   unsigned int* __restrict__ tc_err_bits) {
-    const int32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= nq) return;
+// true neighbour.  A query's candidates are 'lists' lists of list_len entries
+// (32 PER in all at most), each the nearest of its part of the points in
+// ascending FP32 order.  One warp per query, a candidate (or PER) per lane:
+// bound by the candidates' rows, read from L2 a row per lane.  (A thread per
+// query with an insertion sort in local memory took 3.9 ms for a million
+// queries of 24 candidates in 50 dimensions.)
+constexpr int RESCORE_WARPS = 4;
+template <int PER>
+__global__ void __launch_bounds__(RESCORE_WARPS * 32)
+    knn_rescore_kernel(const float* __restrict__ data, int32_t others, int32_t dim, int32_t k,
+                       const int32_t* __restrict__ queries, int32_t nq, int lists, int list_len, int cand_by_slot,
+                       int out_by_slot, const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_d2,
+                       int32_t* __restrict__ out_idx, float* __restrict__ out_dist, double* __restrict__ out_dist64,
+                       int32_t* __restrict__ redo, int32_t* __restrict__ redo_count, const float* __restrict__ norms,
+                       const unsigned int* __restrict__ norm_max_bits, double tc_rel,
+                       unsigned int* __restrict__ tc_err_bits) {
+    const int lane = threadIdx.x & 31;
+    const int64_t slot64 = static_cast<int64_t>(blockIdx.x) * RESCORE_WARPS + (threadIdx.x >> 5);
+    if (slot64 >= nq) return;   // whole warps
+    const int32_t slot = static_cast<int32_t>(slot64);
     const int32_t q = queries ? queries[slot] : slot;     // the query's data row (output row)
-    const size_t crow = static_cast<size_t>(cand_by_slot ? slot : q);   // its candidate list
-    double d64[KCAP];
-    int id[KCAP];
-    const int32_t* ci = cand_idx + crow * KCAP;
+    const int ncand = lists * list_len;
+    const size_t first = static_cast<size_t>(cand_by_slot ? slot : q) * ncand;   // its candidates
     const float* xq = data + static_cast<size_t>(q) * dim;
-    int m = 0;
+    const bool vec4 = dim % 4 == 0 && reinterpret_cast<uintptr_t>(data) % 16 == 0;
+    const double scale = norms ? static_cast<double>(norms[q]) + static_cast<double>(__uint_as_float(*norm_max_bits)) : 0.0;
+    const double err_scale = norms && tc_err_bits ? 1.0 / (scale + 1e-300) : 0.0;
+    double d64[PER];
+    int id[PER];
     float worst = 0.0f;   // largest |FP32 candidate distance - FP64 distance| / (|q|^2 + max |r|^2)
-    const double err_scale = (norms && tc_err_bits)
-                                 ? 1.0 / (static_cast<double>(norms[q]) + static_cast<double>(__uint_as_float(*norm_max_bits)) + 1e-300)
-                                 : 0.0;
-    for (int c = 0; c < KCAP; ++c) {
-        const int32_t j = ci[c];
-        double s = 0;
-        if (j >= 0) {
-            const float* xj = data + static_cast<size_t>(j) * dim;
-            for (int d = 0; d < dim; ++d) {
-                const double diff = static_cast<double>(xq[d]) - static_cast<double>(xj[d]);
-                s = __dadd_rn(s, __dmul_rn(diff, diff));
-            }
-            if (err_scale > 0.0) {
-                const double e = fabs(static_cast<double>(cand_d2[crow * KCAP + c]) - s) * err_scale;
-                worst = fmaxf(worst, static_cast<float>(e));
-            }
-        } else {
-            s = CUDART_INF;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = 32 * i + lane;
+        id[i] = c < ncand ? cand_idx[first + c] : -1;
+        d64[i] = CUDART_INF;
+        if (id[i] >= 0) {
+            d64[i] = distance2(xq, data + static_cast<size_t>(id[i]) * dim, dim, vec4);
+            if (err_scale > 0.0)
+                worst = fmaxf(worst, static_cast<float>(fabs(static_cast<double>(cand_d2[first + c]) - d64[i]) * err_scale));
         }
-        // insertion by (distance, index); empty slots (j < 0) carry +inf and sort last
-        const uint32_t jkey = static_cast<uint32_t>(j);   // -1 maps above every index
-        int pos = m++;
-        while (pos > 0 && (s < d64[pos - 1] || (s == d64[pos - 1] && jkey < static_cast<uint32_t>(id[pos - 1])))) {
-            d64[pos] = d64[pos - 1];
-            id[pos] = id[pos - 1];
-            --pos;
-        }
-        d64[pos] = s;
-        id[pos] = j;
     }
-    // Certainty check: every point outside the candidate list has FP32 distance
-    // >= the list's last FP32 value.  FP32 squared distances from differences
-    // carry relative error below (dim + 2) * 2^-24 (plus the rounding of the
-    // inputs, which is exact here); if the k-th FP64 distance could exceed the
-    // true distance of such a point, the query is recomputed in FP64.
-    // For tensor-core candidates (norms given) the FP32 values are
+    warp_sort<PER>(d64, id);
+    // Certainty check: every point outside the candidate lists has an FP32
+    // distance >= the last FP32 value of its list.  FP32 squared distances from
+    // differences carry relative error below (dim + 2) * 2^-24 (plus the
+    // rounding of the inputs, which is exact here); if the k-th FP64 distance
+    // could exceed the true distance of such a point, the query is recomputed
+    // in FP64.  For tensor-core candidates (norms given) the FP32 values are
     // |q|^2 + |r|^2 - 2 q.r with an absolute error below tc_rel * (|q|^2 + max |r|^2).
-    const float last32 = cand_d2[crow * KCAP + KCAP - 1];
-    const double rel = (dim + 2) * 1.2e-7 * 2.0;
-    const double kth = d64[k - 1];
-    const bool full_list = others <= KCAP;   // every candidate point is in the list
-    bool certain;
-    if (norms) {
-        const double bound = tc_rel * (static_cast<double>(norms[q]) + static_cast<double>(__uint_as_float(*norm_max_bits)));
-        certain = static_cast<double>(last32) - bound > kth * (1.0 + 1e-12) + 1e-300;
-    } else {
-        certain = static_cast<double>(last32) * (1.0 - rel) > kth * (1.0 + rel);
+    float last32 = CUDART_INF_F;
+    for (int l = 0; l < lists; ++l) last32 = fminf(last32, cand_d2[first + (l + 1) * list_len - 1]);
+    double kth = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const double v = __shfl_sync(0xffffffffu, d64[i], (k - 1) & 31);
+        if (i == (k - 1) >> 5) kth = v;
     }
-    if (!full_list && !certain) {
+    const double rel = (dim + 2) * 1.2e-7 * 2.0;
+    const bool full_list = lists == 1 && others <= ncand;   // every candidate point is in the list
+    const bool certain = norms ? static_cast<double>(last32) - tc_rel * scale > kth * (1.0 + 1e-12) + 1e-300
+                               : static_cast<double>(last32) * (1.0 - rel) > kth * (1.0 + rel);
+    if (lane == 0 && !full_list && !certain) {
         const int32_t r = atomicAdd(redo_count, 1);
         redo[r] = out_by_slot ? slot : q;   // a slot when the output is by slot, else the data row
     }
-    if (err_scale > 0.0 && worst > 0.0f) atomicMax(tc_err_bits, __float_as_uint(worst));
-    const size_t orow = static_cast<size_t>(out_by_slot ? slot : q);
-    for (int c = 0; c < k; ++c) {
-        out_idx[orow * k + c] = id[c];
-        const double dd = sqrt(d64[c]);
-        out_dist[orow * k + c] = static_cast<float>(dd);
-        if (out_dist64) out_dist64[orow * k + c] = dd;
+    if (err_scale > 0.0) {
+        for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+        if (lane == 0 && worst > 0.0f) atomicMax(tc_err_bits, __float_as_uint(worst));
+    }
+    const size_t orow = static_cast<size_t>(out_by_slot ? slot : q) * k;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int c = 32 * i + lane;
+        if (c < k) {
+            out_idx[orow + c] = id[i];
+            const double dd = sqrt(d64[i]);
+            out_dist[orow + c] = static_cast<float>(dd);
+            if (out_dist64) out_dist64[orow + c] = dd;
+        }
     }
 }
+
+unsigned rescore_grid(int32_t nq) { return static_cast<unsigned>((nq + RESCORE_WARPS - 1) / RESCORE_WARPS); }
+template <int KCAP>
+constexpr int per_lane() { return (KCAP + 31) / 32; }
 
 // Writes the first k entries of FP64 candidate lists (sqrt of squared distance).
 // Output row of entry 'slot': out_rows[slot] if given, else the query's data row.
@@ -331,8 +404,14 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
         err.zero(s);
         // unsharded: the rows in tree order, so that the rescoring walks the
         // queries with nearby ones together (their candidates share L2 lines)
-        tc = knn_tc_candidates(data, n, dim, KCAP, ci.get(), cd.get(), norms.get(), err.get(), s, shard, rows, nrows,
-                               sharded ? nullptr : &tree_rows);
+        try {
+            tc = knn_tc_candidates(data, n, dim, KCAP, ci.get(), cd.get(), norms.get(), err.get(), s, shard, rows, nrows,
+                                   sharded ? nullptr : &tree_rows);
+        } catch (const Error& e) {
+            // beyond 32 candidates the CUDA-core search, which needs no operands, does where memory is short
+            if (e.code != UMAPB_ERR_OOM || KCAP <= 32) throw;
+            tc = false;
+        }
         int h_err = 0;
         UMAPB_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
         UMAPB_SYNC(s);
@@ -376,10 +455,10 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
     DevArray<unsigned int> tc_err(1, s);
     tc_err.zero(s);
     if (nq > 0) {
-        knn_rescore_kernel<KCAP><<<(nq + 127) / 128, 128, 0, s>>>(data, n - 1, dim, k, queries, nq, by_slot ? 1 : 0, 0, ci.get(),
-                                                                  cd.get(), out_idx, out_dist, out_dist64, redo.get(),
-                                                                  redo_count.get(), tc ? norms.get() : nullptr,
-                                                                  norm_max.get(), TC_REL_BOUND, tc_err.get());
+        knn_rescore_kernel<per_lane<KCAP>()><<<rescore_grid(nq), RESCORE_WARPS * 32, 0, s>>>(
+            data, n - 1, dim, k, queries, nq, 1, KCAP, by_slot ? 1 : 0, 0, ci.get(), cd.get(), out_idx, out_dist,
+            out_dist64, redo.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(), TC_REL_BOUND,
+            tc_err.get());
     }
     UMAPB_LAUNCH_CHECK();
     int32_t nredo = 0;
@@ -444,11 +523,9 @@ void run_f32_batched(const float* data, const std::vector<int32_t>& inst, int32_
     redo_count.zero(s);
     DevArray<unsigned int> tc_err(1, s);
     tc_err.zero(s);
-    knn_rescore_kernel<KCAP><<<(n + 127) / 128, 128, 0, s>>>(data, n - 1, dim, k, nullptr, n, 0, 0, ci.get(), cd.get(),
-                                                             out_idx,
-                                                             out_dist,
-                                                             nullptr, redo.get(), redo_count.get(), norms.get(),
-                                                             norm_max.get(), TC_REL_BOUND, tc_err.get());
+    knn_rescore_kernel<per_lane<KCAP>()><<<rescore_grid(n), RESCORE_WARPS * 32, 0, s>>>(
+        data, n - 1, dim, k, nullptr, n, 1, KCAP, 0, 0, ci.get(), cd.get(), out_idx, out_dist, nullptr, redo.get(),
+        redo_count.get(), norms.get(), norm_max.get(), TC_REL_BOUND, tc_err.get());
     UMAPB_LAUNCH_CHECK();
     int32_t nredo = 0;
     unsigned int err_bits = 0;
@@ -554,29 +631,78 @@ template void knn_exact_shard<float>(const float*, int32_t, int32_t, int32_t, Kn
 template void knn_exact_shard<double>(const double*, int32_t, int32_t, int32_t, KnnShard, int32_t*, double*,
                                       DevArray<int32_t>&, int32_t&, cudaStream_t);
 
+// Ranges the references are split into for nq queries: enough that the query
+// tiles' CTAs fill the device twice over, as many as four lists of KCAP
+// candidates go through one rescoring; 0 where the references are too few for
+// the tensor-core search to pay (10 and 500 queries, 10 and 50 dimensions: 512
+// references 0.24 and 0.27 ms against 0.18 and 0.31 on CUDA cores, 1024 0.23 and
+// 0.28 against 0.25 and 0.49; 100,000 references and 10,000 queries 2.9 against
+// 30 ms).
+static int query_lists(int32_t nref, int32_t nq, int kcap) {
+    if (nref < 1024) return 0;
+    const int64_t tiles = (static_cast<int64_t>(nq) + 127) / 128;
+    int lists = 1;
+    while (lists < 4 && 2 * lists * kcap <= 128 && tiles * lists < 2 * 148) lists *= 2;
+    return lists;
+}
+
 __global__ void add_offset_kernel(int32_t count, const int32_t* __restrict__ src, int32_t add,
                                   int32_t* __restrict__ dst) {
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) dst[i] = src[i] + add;
 }
 
-// Float queries against reference rows: FP32 brute-force candidates (from
-// differences), FP64 rescoring and certification, FP64 search of the
-// uncertain queries.  rows[slot] = nref + slot are the queries' data rows;
-// results are written by slot.
+// Float queries against reference rows: FP32 candidates, FP64 rescoring and
+// certification, FP64 search of the uncertain queries.  rows[slot] = nref +
+// slot are the queries' data rows; results are written by slot.
+// The candidates come from the tensor-core search (knn_tc.cu: every query tile
+// against all references, a query tile's references split over several CTAs
+// with a list each) where it takes the data, else from the brute-force kernel.
 template <int KCAP>
 void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int32_t k, const int32_t* rows,
                    int32_t* out_idx, float* out_dist, cudaStream_t s) {
-    DevArray<int32_t> ci(static_cast<size_t>(nq) * KCAP, s);
-    DevArray<float> cd(static_cast<size_t>(nq) * KCAP, s);
-    knn_bruteforce_kernel<float, float, KCAP><<<(nq + KNN_BLOCK - 1) / KNN_BLOCK, KNN_BLOCK, 0, s>>>(
-        data, nref, dim, rows, nq, ci.get(), cd.get());
-    UMAPB_LAUNCH_CHECK();
+    const int lists = query_lists(nref, nq, KCAP);
+    DevArray<int32_t> ci(static_cast<size_t>(nq) * lists * KCAP, s);
+    DevArray<float> cd(static_cast<size_t>(nq) * lists * KCAP, s);
+    DevArray<float> norms;
+    DevArray<unsigned int> norm_max(1, s);
+    bool tc = use_tensor_cores() && lists > 0 && knn_tc_supported(dim, KCAP);
+    if (tc) {
+        norms.allocate(static_cast<size_t>(nref) + nq, s);
+        DevArray<int> err(1, s);
+        err.zero(s);
+        try {
+            tc = knn_tc_query_candidates(data, nref, nq, dim, KCAP, lists, ci.get(), cd.get(), norms.get(), err.get(), s);
+        } catch (const Error& e) {
+            if (e.code != UMAPB_ERR_OOM) throw;   // the CUDA-core search needs no operands
+            tc = false;
+        }
+        int h_err = 0;
+        UMAPB_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+        UMAPB_SYNC(s);
+        if (h_err != DEV_OK) fail(UMAPB_ERR_DEVICE_TIMEOUT, "tensor-core kNN: a pipeline wait gave up");
+        if (tc) {
+            norm_max.zero(s);
+            norm_max_kernel<<<grid_for(nref + nq, 256, 1024), 256, 0, s>>>(nref + nq, norms.get(), norm_max.get());
+            UMAPB_LAUNCH_CHECK();
+        }
+    }
+    if (!tc) {
+        ci.reserve(static_cast<size_t>(nq) * KCAP, s);
+        cd.reserve(static_cast<size_t>(nq) * KCAP, s);
+        knn_bruteforce_kernel<float, float, KCAP><<<(nq + KNN_BLOCK - 1) / KNN_BLOCK, KNN_BLOCK, 0, s>>>(
+            data, nref, dim, rows, nq, ci.get(), cd.get());
+        UMAPB_LAUNCH_CHECK();
+    }
     DevArray<int32_t> redo(nq, s), redo_count(1, s);
     redo_count.zero(s);
-    knn_rescore_kernel<KCAP><<<(nq + 127) / 128, 128, 0, s>>>(data, nref, dim, k, rows, nq, 1, 1, ci.get(), cd.get(),
-                                                              out_idx, out_dist, nullptr, redo.get(), redo_count.get(),
-                                                              nullptr, nullptr, TC_REL_BOUND, nullptr);
-    UMAPB_LAUNCH_CHECK();
+    auto rescore = [&](auto per) {
+        knn_rescore_kernel<decltype(per)::value><<<rescore_grid(nq), RESCORE_WARPS * 32, 0, s>>>(
+            data, nref, dim, k, rows, nq, tc ? lists : 1, KCAP, 1, 1, ci.get(), cd.get(), out_idx, out_dist, nullptr,
+            redo.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(), TC_REL_BOUND, nullptr);
+        UMAPB_LAUNCH_CHECK();
+    };
+    if (tc && lists * KCAP > 32 * per_lane<KCAP>()) rescore(std::integral_constant<int, 4>());
+    else rescore(std::integral_constant<int, per_lane<KCAP>()>());
     int32_t nredo = 0;
     UMAPB_CUDA(cudaMemcpyAsync(&nredo, redo_count.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     UMAPB_SYNC(s);

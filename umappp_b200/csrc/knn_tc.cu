@@ -553,7 +553,7 @@ bool knn_tc_supported(int32_t dim, int kcap) {
 static float f16_scale_or_zero(const float* data, size_t count, int32_t dim, int kcap, cudaStream_t s) {
     if (!use_f16_operands() || !knn_tc16_supported(dim, kcap)) return 0.0f;
     const float scale = knn_tc16_scale(data, count, s);
-    require(scale > 0.0f || tf32_supported(dim, kcap),
+    require(scale > 0.0f || tf32_supported(dim, kcap) || kcap > 32,
             "tensor-core kNN: the data have no finite maximum in [2^-60, 2^60] for the FP16 search");
     return scale;
 }
@@ -572,10 +572,28 @@ bool knn_tc_candidates(const float* data, int32_t n, int32_t dim, int kcap, int3
                        shard_count, tree_rows);
         return true;
     }
+    if (!tf32_supported(dim, kcap)) return false;   // more than 32 candidates and no scale: the caller searches on CUDA cores
     if (shard.count > 1) return false;   // the TF32 search covers every query: the caller shards by rows instead
     last_knn_tiles_scanned() = static_cast<int64_t>(n_pad / TC_M) * (n_pad / TC_N);
     run_candidates(data, n, dim, kcap, n_pad, nullptr, n_pad / TC_M, nullptr, nullptr, cand_idx, cand_d2, norms_out,
                    d_err, s);
+    return true;
+}
+
+// Candidates of the queries [nref, nref + nq) among the references [0, nref):
+// 'lists' lists of kcap per query (row - nref), each the nearest of a range of
+// the references; false, computing nothing, when the data have no scale for
+// the FP16 search.  norms_out receives |x|^2 of every data row.
+bool knn_tc_query_candidates(const float* data, int32_t nref, int32_t nq, int32_t dim, int kcap, int32_t lists,
+                             int32_t* cand_idx, float* cand_d2, float* norms_out, int* d_err, cudaStream_t s) {
+    if (!use_f16_operands() || !knn_tc16_supported(dim, kcap)) return false;
+    const float scale = knn_tc16_scale(data, (static_cast<size_t>(nref) + nq) * dim, s);
+    if (!(scale > 0.0f)) return false;
+    KnnTiles tiles;
+    KnnTasks tasks;
+    knn_query_tasks(nref, nq, lists, tiles, tasks, s);
+    knn_tc16_run_tasks(data, dim, kcap, scale, tiles, tasks, cand_idx, cand_d2, norms_out, d_err, s, nullptr, 12);
+    UMAPB_SYNC(s);   // the tile and task buffers are released below
     return true;
 }
 

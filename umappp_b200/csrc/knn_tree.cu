@@ -267,7 +267,7 @@ __global__ void group_bounds_kernel(const float* __restrict__ data, int32_t dim,
     }
 }
 
-constexpr int KTH_MAX = 32;
+constexpr int KTH_MAX = 64;
 constexpr float D2_LOW = 1.0f - 1.0e-4f;    // lower-bound factor on FP32 squared distances
 constexpr float D2_HIGH = 1.0f + 1.0e-4f;   // upper-bound factor
 
@@ -648,6 +648,7 @@ void knn_tile_tasks(const float* data, int32_t dim, const KnnTiles& t, const std
         };
         if (k <= 16) launch(std::integral_constant<int, 16>());
         else if (k <= 24) launch(std::integral_constant<int, 24>());
+        else if (k <= 32) launch(std::integral_constant<int, 32>());
         else launch(std::integral_constant<int, KTH_MAX>());
         UMAPB_LAUNCH_CHECK();
     }
@@ -700,6 +701,38 @@ void knn_tile_tasks(const float* data, int32_t dim, const KnnTiles& t, const std
     out.host_tasks = sorted;
     out.tasks.allocate(std::max<size_t>(sorted.size(), 1), s);
     UMAPB_CUDA(cudaMemcpyAsync(out.tasks.get(), sorted.data(), sorted.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+    UMAPB_SYNC(s);   // host vectors above
+}
+
+void knn_query_tasks(int32_t nref, int32_t nq, int32_t lists, KnnTiles& tiles, KnnTasks& out, cudaStream_t s) {
+    knn_tree_order(nullptr, 0, {0, nref, nref + nq}, false, tiles, s);
+    const int32_t rtiles = tiles.pad_start[1] / TREE_LEAF, qtiles = tiles.pad_start[2] / TREE_LEAF - rtiles;
+    std::vector<int4> tasks;
+    std::vector<int64_t> off;
+    std::vector<int32_t> len, list(rtiles);
+    for (int32_t x = 0; x < rtiles; ++x) list[x] = x;
+    for (int32_t q = 0; q < qtiles; ++q) {
+        for (int32_t l = 0; l < lists; ++l) {
+            const int32_t a = static_cast<int32_t>(static_cast<int64_t>(rtiles) * l / lists);
+            const int32_t b = static_cast<int32_t>(static_cast<int64_t>(rtiles) * (l + 1) / lists);
+            // a query tile of its own for every range: one task per list
+            tasks.push_back(make_int4((rtiles + q) * TREE_LEAF, static_cast<int32_t>(tasks.size()), 1, l));
+            off.push_back(a);
+            len.push_back(b - a);
+        }
+    }
+    out.count = static_cast<int32_t>(tasks.size());
+    out.total_tiles = static_cast<int64_t>(qtiles) * rtiles;
+    out.out_row0 = nref;
+    out.lists = lists;
+    out.tasks.allocate(tasks.size(), s);
+    out.qlist_off.allocate(off.size(), s);
+    out.qlist_len.allocate(len.size(), s);
+    out.tile_list.allocate(list.size(), s);
+    UMAPB_CUDA(cudaMemcpyAsync(out.tasks.get(), tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+    UMAPB_CUDA(cudaMemcpyAsync(out.qlist_off.get(), off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    UMAPB_CUDA(cudaMemcpyAsync(out.qlist_len.get(), len.data(), len.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+    UMAPB_CUDA(cudaMemcpyAsync(out.tile_list.get(), list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     UMAPB_SYNC(s);   // host vectors above
 }
 

@@ -65,6 +65,8 @@ bool knn_tc_candidates(const float* data, int32_t n, int32_t dim, int kcap, int3
                        float* norms_out, int* d_err, cudaStream_t s, KnnShard shard = KnnShard(),
                        DevArray<int32_t>* shard_rows = nullptr, int32_t* shard_count = nullptr,
                        DevArray<int32_t>* tree_rows = nullptr);
+bool knn_tc_query_candidates(const float* data, int32_t nref, int32_t nq, int32_t dim, int kcap, int32_t lists,
+                             int32_t* cand_idx, float* cand_d2, float* norms_out, int* d_err, cudaStream_t s);
 // Batched: instance i is data rows [inst[i], inst[i + 1]) (host vector).
 void knn_tc_candidates_batched(const float* data, const std::vector<int32_t>& inst, int32_t dim, int kcap,
                                int32_t* cand_idx, float* cand_d2, int* d_err, cudaStream_t s);
@@ -79,12 +81,13 @@ struct KnnTiles {
     int32_t n_pad = 0;
 };
 struct KnnTasks {
-    DevArray<int4> tasks;          // per CTA: {first operand row, first query tile, query tiles, 0}
+    DevArray<int4> tasks;          // per CTA: {first operand row, first query tile, query tiles, list}
     DevArray<int64_t> qlist_off;   // per query tile: its reference tiles are
     DevArray<int32_t> qlist_len;   //   tile_list[qlist_off .. + qlist_len)
     DevArray<int32_t> tile_list;
     int32_t count = 0;
     int64_t total_tiles = 0;       // sum of the query tiles' list lengths
+    int32_t out_row0 = 0, lists = 1;   // data row of the first output row; candidate lists per row (one per task of its tile)
     std::vector<int4> host_tasks;  // the tasks, in launch order
 };
 // Data rows of the query tiles of a task list (ascending): the rows a sharded
@@ -94,6 +97,10 @@ void knn_tree_rows(const KnnTiles& t, int32_t n, DevArray<int32_t>& rows, cudaSt
 void knn_task_rows(const KnnTiles& t, const KnnTasks& tk, int32_t n, DevArray<int32_t>& rows, int32_t& count,
                    cudaStream_t s);
 // tree == false keeps each instance in data order.
+// The queries [nref, nref + nq) against the references [0, nref) of 'data':
+// operand order, and tasks that split the references into 'lists' ranges per
+// query tile.
+void knn_query_tasks(int32_t nref, int32_t nq, int32_t lists, KnnTiles& tiles, KnnTasks& out, cudaStream_t s);
 void knn_tree_order(const float* data, int32_t dim, const std::vector<int32_t>& inst, bool tree, KnnTiles& out,
                     cudaStream_t s);
 // Every query tile lists the reference tiles of its instance that may hold one
