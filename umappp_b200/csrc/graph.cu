@@ -356,19 +356,23 @@ __global__ void uf_init_kernel(int32_t n, int32_t* parent) {
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) parent[i] = i;
 }
 
+constexpr int HOOK_LANES = 8;
+
 // Hooks the larger root under the smaller one.  Roots only ever point to
 // smaller indices, so the loop makes progress; it is still capped, and a cap
 // hit is reported through the status word.
 __global__ void uf_hook_kernel(int32_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                int32_t* parent, int* status) {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        for (int64_t p = ptr[i]; p < ptr[i + 1]; ++p) {
+    // HOOK_LANES threads per row
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x / HOOK_LANES;
+    for (int64_t i = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / HOOK_LANES; i < n; i += step) {
+        for (int64_t p = ptr[i] + threadIdx.x % HOOK_LANES; p < ptr[i + 1]; p += HOOK_LANES) {
             const int32_t j = idx[p];
             if (j < 0 || j >= n) {
                 atomicExch(status, DEV_BAD_INPUT);
                 continue;
             }
-            int32_t a = i, b = j;
+            int32_t a = static_cast<int32_t>(i), b = j;
             bool done = false;
             for (int iter = 0; iter < (1 << 20) && !done; ++iter) {
                 a = uf_find(parent, a);
@@ -405,7 +409,7 @@ int64_t count_components(int32_t n, const int64_t* ptr, const int32_t* idx, int*
     UMAPB_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
     uf_init_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, parent.get());
     UMAPB_LAUNCH_CHECK();
-    uf_hook_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, ptr, idx, parent.get(), d_status);
+    uf_hook_kernel<<<grid_for(static_cast<size_t>(n) * HOOK_LANES, 256), 256, 0, s>>>(n, ptr, idx, parent.get(), d_status);
     UMAPB_LAUNCH_CHECK();
     uf_count_roots_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, parent.get(), count.get());
     UMAPB_LAUNCH_CHECK();

@@ -33,30 +33,166 @@ __global__ void degree_sqrt_kernel(int32_t n, const int64_t* __restrict__ ptr, c
     }
 }
 
+// One warp per row: rows differ in length by a factor of a hundred.
 template <typename T>
 __global__ void laplacian_values_kernel(int32_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                         const T* __restrict__ w, const double* __restrict__ sums,
                                         double* __restrict__ lap) {
-    for (int32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        for (int64_t p = ptr[c]; p < ptr[c + 1]; ++p) {
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t c = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n; c += warps) {
+        for (int64_t p = ptr[c] + (threadIdx.x & 31); p < ptr[c + 1]; p += 32) {
             lap[p] = __dmul_rn(__ddiv_rn(__ddiv_rn(-static_cast<double>(w[p]), sums[idx[p]]), sums[c]), -1.0);
         }
     }
 }
 
-// y = (I + D^-1/2 W D^-1/2) x, each row summed in stored order with the unit
-// diagonal at its sorted position (the compressed layout of :60-78).
-__global__ void lap_spmv_kernel(int32_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                                const double* __restrict__ lap, const double* __restrict__ x, double* __restrict__ y) {
-    for (int32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        int64_t p = ptr[c];
-        const int64_t e = ptr[c + 1];
+// ---- Lanczos steps ----
+// One step is three launches without a host read: every block owns a stretch
+// of rows, so a product's rows go into the block's part of the next dot
+// products at once, and a sum over blocks is taken by every block of the next
+// launch for itself (the same bits everywhere).
+//   step_product    v_j = x / |x| (its norm's partial sums given), w = A v_j,
+//                   partial dots of w with v_0 .. v_j
+//   step_project    w -= V h, then the partial dots again (first pass) or the
+//                   partial squared norm (second pass)
+// At 20,000 points a step takes 31 us; a row per thread and a launch for each
+// vector operation, with two host reads, took 140 us (76 of them the product:
+// its longest row is 300 edges).
+constexpr int STEP_BLOCK = 512;
+constexpr int STEP_WARPS = STEP_BLOCK / 32;
+constexpr int MAX_BASIS = 64;
+
+__device__ __forceinline__ double warp_sum(double x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Sums of the blocks' partials of column c (nblk of them), by one warp.
+__device__ __forceinline__ double sum_partials(const double* __restrict__ partial, int c, int nblk) {
+    double s = 0;
+    for (int b = threadIdx.x & 31; b < nblk; b += 32) s += partial[static_cast<size_t>(c) * nblk + b];
+    return warp_sum(s);
+}
+
+// This block's rows of an n-vector.
+__device__ __forceinline__ void block_rows(int32_t n, int32_t& r0, int32_t& r1) {
+    r0 = static_cast<int32_t>(static_cast<int64_t>(n) * blockIdx.x / gridDim.x);
+    r1 = static_cast<int32_t>(static_cast<int64_t>(n) * (blockIdx.x + 1) / gridDim.x);
+}
+
+// partial[c][block] = the block's part of V[:, c] . w, c < ncol; w's rows of
+// this block are complete.
+__device__ __forceinline__ void partial_dots(int32_t n, int32_t r0, int32_t r1, const double* V, int ncol,
+                                             const double* w, double* __restrict__ partial) {
+    const int lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < ncol; c += STEP_WARPS) {
+        const double* v = V + static_cast<size_t>(c) * n;
         double s = 0;
-        for (; p < e && idx[p] < c; ++p) s = __dadd_rn(s, __dmul_rn(lap[p], x[idx[p]]));
-        s = __dadd_rn(s, x[c]);
-        for (; p < e; ++p) s = __dadd_rn(s, __dmul_rn(lap[p], x[idx[p]]));
-        y[c] = s;
+        for (int32_t i = r0 + lane; i < r1; i += 32) s += v[i] * w[i];
+        s = warp_sum(s);
+        if (lane == 0) partial[static_cast<size_t>(c) * gridDim.x + blockIdx.x] = s;
     }
+}
+
+// x: v_j itself (norm2 null: then it is column j already), or a vector whose
+// squared norm's partials are norm2; it is scaled to unit length (to zero if it
+// is zero) and becomes column j, its norm *beta.  w = (I + D^-1/2 W D^-1/2) v_j.
+__global__ void __launch_bounds__(STEP_BLOCK, 2)
+    step_product_kernel(int32_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                        const double* __restrict__ lap, const double* __restrict__ x, const double* __restrict__ norm2,
+                        double* V, int j, double* w, double* __restrict__ partial, double* __restrict__ beta) {
+    __shared__ double scale;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t r0, r1;
+    block_rows(n, r0, r1);
+    double* vj = V + static_cast<size_t>(j) * n;
+    if (warp == 0) {
+        double f = 1.0;
+        if (norm2) {
+            const double nrm = sqrt(sum_partials(norm2, 0, gridDim.x));
+            f = nrm > 0 ? 1.0 / nrm : 0.0;
+            if (blockIdx.x == 0 && lane == 0) *beta = nrm;
+        }
+        if (lane == 0) scale = f;
+    }
+    __syncthreads();
+    const double f = scale;
+    if (norm2)
+        for (int32_t i = r0 + threadIdx.x; i < r1; i += STEP_BLOCK) vj[i] = x[i] * f;
+    for (int32_t c = r0 + warp; c < r1; c += STEP_WARPS) {
+        double s = 0;
+        for (int64_t p = ptr[c] + lane; p < ptr[c + 1]; p += 32) s += lap[p] * (x[idx[p]] * f);
+        s = warp_sum(s);
+        if (lane == 0) w[c] = x[c] * f + s;
+    }
+    __syncthreads();
+    partial_dots(n, r0, r1, V, j + 1, w, partial);
+}
+
+// The dots alone (a fresh direction after an invariant subspace).
+__global__ void __launch_bounds__(STEP_BLOCK, 2)
+    step_dots_kernel(int32_t n, const double* V, int ncol, const double* w, double* __restrict__ partial) {
+    int32_t r0, r1;
+    block_rows(n, r0, r1);
+    partial_dots(n, r0, r1, V, ncol, w, partial);
+}
+
+// w -= V[:, :ncol] h, h the sums of 'partial'; then 'out' gets the partial dots
+// of w (second = false) or of |w|^2.  *alpha: h of the last column.
+__global__ void __launch_bounds__(STEP_BLOCK, 2)
+    step_project_kernel(int32_t n, const double* V, int ncol, const double* __restrict__ partial, double* w,
+                        double* __restrict__ out, bool second, double* __restrict__ alpha) {
+    __shared__ double h[MAX_BASIS + 1];
+    __shared__ double red[STEP_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t r0, r1;
+    block_rows(n, r0, r1);
+    for (int c = warp; c < ncol; c += STEP_WARPS) {
+        const double s = sum_partials(partial, c, gridDim.x);
+        if (lane == 0) {
+            h[c] = s;
+            if (blockIdx.x == 0 && c == ncol - 1) *alpha = s;
+        }
+    }
+    __syncthreads();
+    double sq = 0;
+    for (int32_t i = r0 + threadIdx.x; i < r1; i += STEP_BLOCK) {
+        double s = w[i];
+        for (int c = 0; c < ncol; ++c) s -= h[c] * V[static_cast<size_t>(c) * n + i];
+        w[i] = s;
+        sq += s * s;
+    }
+    if (!second) {
+        __syncthreads();
+        partial_dots(n, r0, r1, V, ncol, w, out);
+        return;
+    }
+    sq = warp_sum(sq);
+    if (lane == 0) red[warp] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0;
+        for (int q = 0; q < STEP_WARPS; ++q) s += red[q];
+        out[blockIdx.x] = s;
+    }
+}
+
+// Column 'col' = w / |w| and *beta = |w|, the end of a basis.
+__global__ void __launch_bounds__(STEP_BLOCK, 2)
+    step_scale_kernel(int32_t n, const double* __restrict__ w, const double* __restrict__ norm2, double* __restrict__ col,
+                      double* __restrict__ beta) {
+    __shared__ double scale;
+    int32_t r0, r1;
+    block_rows(n, r0, r1);
+    if (threadIdx.x < 32) {
+        const double nrm = sqrt(sum_partials(norm2, 0, gridDim.x));
+        if (threadIdx.x == 0) {
+            scale = nrm > 0 ? 1.0 / nrm : 0.0;
+            if (blockIdx.x == 0) *beta = nrm;
+        }
+    }
+    __syncthreads();
+    for (int32_t i = r0 + threadIdx.x; i < r1; i += STEP_BLOCK) col[i] = w[i] * scale;
 }
 
 constexpr int DOT_BLOCK = 256;
@@ -80,24 +216,12 @@ __global__ void __launch_bounds__(DOT_BLOCK) multi_dot_kernel(int32_t n, const d
     }
 }
 
-__global__ void reduce_partials_kernel(int nblk, int ncol, const double* __restrict__ partial, double* __restrict__ h,
-                                       double* __restrict__ h_accum) {
+__global__ void reduce_partials_kernel(int nblk, int ncol, const double* __restrict__ partial, double* __restrict__ h) {
     const int c = threadIdx.x;
     if (c >= ncol) return;
     double t = 0;
     for (int b = 0; b < nblk; ++b) t += partial[static_cast<size_t>(b) * ncol + c];
     h[c] = t;
-    if (h_accum) h_accum[c] += t;
-}
-
-// w -= V[:, :ncol] h
-__global__ void subtract_projection_kernel(int32_t n, const double* __restrict__ V, int ncol,
-                                           const double* __restrict__ h, double* __restrict__ w) {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double s = w[i];
-        for (int c = 0; c < ncol; ++c) s -= h[c] * V[static_cast<size_t>(c) * n + i];
-        w[i] = s;
-    }
 }
 
 __global__ void scale_vector_kernel(int32_t n, const double* __restrict__ x, double f, double* __restrict__ y) {
@@ -245,7 +369,7 @@ void jacobi_eigen(int m, std::vector<double>& A, std::vector<double>& evals, std
     }
 }
 
-// Lanczos workspace and primitive steps on the device.
+// Lanczos workspace and steps on the device.
 struct LanczosDevice {
     int32_t n;
     int ncv;
@@ -253,40 +377,65 @@ struct LanczosDevice {
     const int64_t* ptr;
     const int32_t* idx;
     const double* lap;
-    DevArray<double> V, h, hsum, partial, tmp;
-    int nblk;
+    DevArray<double> V, h, partial, tmp;
+    DevArray<double> w[2], dots[2], norm2, coef;   // coef: per step, alpha of both passes and beta
+    int nblk, steps_blk;
+    int cur = 0;               // w[cur]: the last step's vector, its squared norm in norm2
 
     LanczosDevice(int32_t n_, int ncv_, const int64_t* p, const int32_t* i, const double* l, cudaStream_t st)
         : n(n_), ncv(ncv_), s(st), ptr(p), idx(i), lap(l) {
         V.allocate(static_cast<size_t>(n) * (ncv + 1), s);
-        h.allocate(ncv + 2, s);
-        hsum.allocate(ncv + 2, s);
+        h.allocate(1, s);
         nblk = static_cast<int>(std::min<int64_t>((n + 1023) / 1024, 256));
-        partial.allocate(static_cast<size_t>(nblk) * (ncv + 2), s);
+        partial.allocate(nblk, s);
         tmp.allocate(static_cast<size_t>(n) * (ncv + 1), s);
+        steps_blk = static_cast<int>(std::min<int64_t>((n + STEP_WARPS - 1) / STEP_WARPS, 2 * 148));
+        for (int b = 0; b < 2; ++b) {
+            w[b].allocate(n, s);
+            dots[b].allocate(static_cast<size_t>(steps_blk) * (ncv + 1), s);
+        }
+        norm2.allocate(steps_blk, s);
+        coef.allocate(3 * (static_cast<size_t>(ncv) + 1), s);
     }
     double* col(int c) const { return V.get() + static_cast<size_t>(c) * n; }
+    // coefficients of step j: h of column j in the two passes, norm of what is left
+    double* alpha1(int j) const { return coef.get() + 3 * j; }
 
-    void matvec(const double* x, double* y) {
-        lap_spmv_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, ptr, idx, lap, x, y);
-        UMAPB_LAUNCH_CHECK();
-    }
-    // two-pass classical Gram-Schmidt of w against columns [0, ncol); hsum gets the coefficients
-    void reorth(double* w, int ncol) {
-        UMAPB_CUDA(cudaMemsetAsync(hsum.get(), 0, sizeof(double) * (ncv + 2), s));
+    // w[cur] made orthogonal to columns [0, ncol) (dots[0] given), its norm in norm2
+    void project(int ncol, int j) {
         for (int pass = 0; pass < 2; ++pass) {
-            multi_dot_kernel<<<dim3(nblk, ncol), DOT_BLOCK, 0, s>>>(n, V.get(), ncol, w, partial.get());
-            UMAPB_LAUNCH_CHECK();
-            reduce_partials_kernel<<<1, 128, 0, s>>>(nblk, ncol, partial.get(), h.get(), hsum.get());
-            UMAPB_LAUNCH_CHECK();
-            subtract_projection_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, V.get(), ncol, h.get(), w);
+            step_project_kernel<<<steps_blk, STEP_BLOCK, 0, s>>>(n, V.get(), ncol, dots[pass].get(), w[cur].get(),
+                                                                 pass ? norm2.get() : dots[1].get(), pass != 0,
+                                                                 alpha1(j) + pass);
             UMAPB_LAUNCH_CHECK();
         }
     }
-    double norm(const double* w) {
-        multi_dot_kernel<<<dim3(nblk, 1), DOT_BLOCK, 0, s>>>(n, w, 1, w, partial.get());
+    // Steps [j, ncv).  ready: column j is there; else it is w[cur], to be scaled.
+    void steps(int j, bool ready) {
+        for (; j < ncv; ++j, ready = false) {
+            const double* x = ready ? col(j) : w[cur].get();
+            cur ^= 1;
+            step_product_kernel<<<steps_blk, STEP_BLOCK, 0, s>>>(n, ptr, idx, lap, x, ready ? nullptr : norm2.get(), V.get(),
+                                                                 j, w[cur].get(), dots[0].get(),
+                                                                 j > 0 ? alpha1(j - 1) + 2 : alpha1(ncv));
+            UMAPB_LAUNCH_CHECK();
+            project(j + 1, j);
+        }
+        step_scale_kernel<<<steps_blk, STEP_BLOCK, 0, s>>>(n, w[cur].get(), norm2.get(), col(ncv), alpha1(ncv - 1) + 2);
         UMAPB_LAUNCH_CHECK();
-        reduce_partials_kernel<<<1, 32, 0, s>>>(nblk, 1, partial.get(), h.get(), nullptr);
+    }
+    // After step j: a fresh direction, orthogonal to columns [0, j], as w[cur].
+    void fresh(int j, uint64_t seed) {
+        start_vector_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, seed, w[cur].get());
+        UMAPB_LAUNCH_CHECK();
+        step_dots_kernel<<<steps_blk, STEP_BLOCK, 0, s>>>(n, V.get(), j + 1, w[cur].get(), dots[0].get());
+        UMAPB_LAUNCH_CHECK();
+        project(j + 1, ncv);   // its coefficients are not part of the projected matrix
+    }
+    double norm(const double* x) {
+        multi_dot_kernel<<<dim3(nblk, 1), DOT_BLOCK, 0, s>>>(n, x, 1, x, partial.get());
+        UMAPB_LAUNCH_CHECK();
+        reduce_partials_kernel<<<1, 32, 0, s>>>(nblk, 1, partial.get(), h.get());
         UMAPB_LAUNCH_CHECK();
         double v = 0;
         UMAPB_CUDA(cudaMemcpyAsync(&v, h.get(), sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -296,12 +445,6 @@ struct LanczosDevice {
     void scale(const double* x, double f, double* y) {
         scale_vector_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, x, f, y);
         UMAPB_LAUNCH_CHECK();
-    }
-    double hsum_at(int c) {
-        double v = 0;
-        UMAPB_CUDA(cudaMemcpyAsync(&v, hsum.get() + c, sizeof(double), cudaMemcpyDeviceToHost, s));
-        UMAPB_SYNC(s);
-        return v;
     }
 };
 
@@ -323,7 +466,7 @@ SpectralResult spectral_init(int32_t n, const int64_t* ptr, const int32_t* idx, 
     DevArray<double> sums(n, s), lap(std::max<int64_t>(nnz, 1), s);
     degree_sqrt_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(n, ptr, w, sums.get());
     UMAPB_LAUNCH_CHECK();
-    laplacian_values_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(n, ptr, idx, w, sums.get(), lap.get());
+    laplacian_values_kernel<T><<<grid_for(static_cast<size_t>(n) * 32, 256), 256, 0, s>>>(n, ptr, idx, w, sums.get(), lap.get());
     UMAPB_LAUNCH_CHECK();
 
     int ncv = nev + std::max(extra_work, nev) + 8;
@@ -346,30 +489,34 @@ SpectralResult spectral_init(int32_t n, const int64_t* ptr, const int32_t* idx, 
     DevArray<double> Sdev(static_cast<size_t>(ncv) * ncv, s);
     const int restarts = std::max(max_iterations, 1);
     for (int restart = 0; restart < restarts; ++restart) {
-        for (int j = k; j < ncv; ++j) {
-            double* vj = L.col(j);
-            double* wv = L.col(j + 1);
-            L.matvec(vj, wv);
-            L.reorth(wv, j + 1);
-            T_[j * ncv + j] = L.hsum_at(j);
-            double beta = L.norm(wv);
-            if (!(beta > 1e-12 * (std::fabs(T_[j * ncv + j]) + 1e-300))) {
-                // invariant subspace: continue from a fresh direction orthogonal to the basis
-                start_vector_kernel<<<grid_for(n, 256), 256, 0, s>>>(
-                    n, start_seed + 7919u * static_cast<uint64_t>(j + 1) + 104729u * static_cast<uint64_t>(restart), wv);
-                UMAPB_LAUNCH_CHECK();
-                L.reorth(wv, j + 1);
-                const double nrm = L.norm(wv);
-                L.scale(wv, nrm > 0 ? 1.0 / nrm : 0.0, wv);   // a full basis leaves nothing to add
-                beta = 0;
-            } else {
-                L.scale(wv, 1.0 / beta, wv);
+        std::vector<double> coef(3 * static_cast<size_t>(ncv));
+        bool ready = true;
+        for (int j = k; j < ncv;) {
+            L.steps(j, ready);
+            UMAPB_CUDA(cudaMemcpyAsync(coef.data(), L.coef.get(), sizeof(double) * coef.size(), cudaMemcpyDeviceToHost, s));
+            UMAPB_SYNC(s);
+            for (ready = true; j < ncv && ready; ++j) {
+                const double alpha = coef[3 * j] + coef[3 * j + 1];
+                double beta = coef[3 * j + 2];
+                T_[j * ncv + j] = alpha;
+                if (!(beta > 1e-12 * (std::fabs(alpha) + 1e-300))) {
+                    // invariant subspace: continue from a fresh direction orthogonal to the basis
+                    // (a full basis leaves nothing to add)
+                    L.fresh(j, start_seed + 7919u * static_cast<uint64_t>(j + 1) + 104729u * static_cast<uint64_t>(restart));
+                    beta = 0;
+                    ready = false;
+                    if (j + 1 == ncv) {
+                        step_scale_kernel<<<L.steps_blk, STEP_BLOCK, 0, s>>>(n, L.w[L.cur].get(), L.norm2.get(), L.col(ncv),
+                                                                             L.alpha1(ncv));
+                        UMAPB_LAUNCH_CHECK();
+                    }
+                }
+                if (j + 1 < ncv) {
+                    T_[j * ncv + j + 1] = beta;
+                    T_[(j + 1) * ncv + j] = beta;
+                }
+                beta_last = beta;
             }
-            if (j + 1 < ncv) {
-                T_[j * ncv + j + 1] = beta;
-                T_[(j + 1) * ncv + j] = beta;
-            }
-            beta_last = beta;
         }
         Tc = T_;
         jacobi_eigen(ncv, Tc, theta, S);
