@@ -28,6 +28,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "pow_pos.cuh"
 #include "stages.cuh"
 #include "umap_grad.cuh"
 
@@ -226,7 +227,7 @@ __device__ __forceinline__ double floor_eps(double d2) {
 template <int NC>
 __device__ __forceinline__ void step_gradient(double d2, bool attract, const double (&diff)[NC],
                                               const StepParams<double>& p, double (&g)[NC]) {
-    const double q = pow(d2, p.b);
+    const double q = pow_pos(d2, p.b);
     const double c = (attract ? p.neg2ab * q : p.gamma2b) / ((attract ? d2 : 0.001 + d2) * (p.a * q + 1.0));
 #pragma unroll
     for (int j = 0; j < NC; ++j) g[j] = c * diff[j];
