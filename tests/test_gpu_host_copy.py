@@ -1,0 +1,45 @@
+"""Pageable host arrays to the device and back (host_copy.cu): a layout that is
+loaded and stored by a run of no epochs comes back as it was, at sizes around
+those where the copy takes another way (1 MiB) and where it starts another slot
+(2 MiB), from one thread and from several at once."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def round_trip(umap, n, seed):
+    Y = np.random.default_rng(seed).integers(0, 2**31, size=(n, 1)).astype(np.int32).view(np.float32)
+    want = Y.copy()
+    none = np.zeros(0, np.float32)
+    ep = umap.EpochData(np.zeros(n + 1, np.int64), np.zeros(0, np.int32), none, none, none, total_epochs=10, current_epoch=3)
+    umap.optimize_layout(1, Y, ep, 1.5, 0.9, 1.0, 1.0, 1, 3, 5.0)
+    assert np.array_equal(Y.view(np.int32), want.view(np.int32))
+
+
+@pytest.mark.parametrize("nbytes", [4, MIB - 4, MIB, MIB + 4, 2 * MIB, 2 * MIB + 4, 8 * MIB, 8 * MIB + 4, 19 * MIB + 12])
+def test_round_trip(umap, nbytes):
+    for seed in range(3):
+        round_trip(umap, nbytes // 4, seed)
+
+
+def test_round_trips_at_once(umap):
+    failures = []
+
+    def work(i):
+        try:
+            for k in range(6):
+                round_trip(umap, (3 + i) * MIB // 4 + 7 * k, 10 * i + k)
+        except BaseException as e:   # noqa: BLE001 - reported below
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures

@@ -318,7 +318,7 @@ void init_from_neighbors(umapb_status* st, const int64_t* row_ptr, const int32_t
     DeviceIn<int64_t> dptr(row_ptr, static_cast<size_t>(n) + 1, s);
     DeviceIn<int32_t> didx(indices, nnz, s);
     DevArray<T> w(nnz, s);
-    if (nnz) UMAPB_CUDA(cudaMemcpyAsync(w.get(), distances, sizeof(T) * nnz, cudaMemcpyDefault, s));
+    if (nnz) copy_async(w.get(), distances, sizeof(T) * nnz, s);
     auto impl = std::make_unique<StatusImpl<T>>(st);
     StageTimer tm(s, st->stage_ms);
     impl->initialize(dptr.get(), didx.get(), w.get(), nnz, embedding, tm);
@@ -392,7 +392,7 @@ void init_from_knn_matrix(umapb_status* st, int32_t k, const int32_t* indices, c
         idx = rebased.get();
     }
     DevArray<T> w(nnz, s);   // consumed (turned into weights)
-    if (nnz) UMAPB_CUDA(cudaMemcpyAsync(w.get(), distances, sizeof(T) * nnz, cudaMemcpyDefault, s));
+    if (nnz) copy_async(w.get(), distances, sizeof(T) * nnz, s);
     DevArray<int64_t> ptr(static_cast<size_t>(n) + 1, s);
     dense_row_ptr_kernel<<<grid_for(static_cast<size_t>(n) + 1, 256), 256, 0, s>>>(n, k, ptr.get());
     UMAPB_LAUNCH_CHECK();
@@ -848,9 +848,9 @@ int umapb_knn_shard(int dtype, size_t data_dim, int32_t num_obs, const void* dat
                     nrows, k, rows.get(), dist.get(), cdist.get());
                 UMAPB_LAUNCH_CHECK();
                 require(out_rows && out_indices && out_distances, "output arrays must not be NULL");
-                UMAPB_CUDA(cudaMemcpyAsync(out_rows, rows.get(), sizeof(int32_t) * nrows, cudaMemcpyDefault, s));
-                UMAPB_CUDA(cudaMemcpyAsync(out_indices, cidx.get(), sizeof(int32_t) * nrows * k, cudaMemcpyDefault, s));
-                UMAPB_CUDA(cudaMemcpyAsync(out_distances, cdist.get(), sizeof(T) * nrows * k, cudaMemcpyDefault, s));
+                copy_async(out_rows, rows.get(), sizeof(int32_t) * nrows, s);
+                copy_async(out_indices, cidx.get(), sizeof(int32_t) * nrows * k, s);
+                copy_async(out_distances, cdist.get(), sizeof(T) * nrows * k, s);
             }
             UMAPB_SYNC(s);
             *out_count = nrows;
@@ -1093,12 +1093,12 @@ int umapb_optimize_layout(int dtype, size_t num_dim, void* embedding, int32_t nu
             ep.eps.allocate(nnz, c.stream);
             ep.enext0.allocate(nnz, c.stream);
             ep.enneg0.allocate(nnz, c.stream);
-            UMAPB_CUDA(cudaMemcpyAsync(ep.ptr.get(), row_ptr, sizeof(int64_t) * (num_obs + 1), cudaMemcpyDefault, c.stream));
+            copy_async(ep.ptr.get(), row_ptr, sizeof(int64_t) * (num_obs + 1), c.stream);
             if (nnz) {
-                UMAPB_CUDA(cudaMemcpyAsync(ep.targets.get(), targets, sizeof(int32_t) * nnz, cudaMemcpyDefault, c.stream));
-                UMAPB_CUDA(cudaMemcpyAsync(ep.eps.get(), epochs_per_sample, sizeof(T) * nnz, cudaMemcpyDefault, c.stream));
-                UMAPB_CUDA(cudaMemcpyAsync(ep.enext0.get(), epoch_of_next_sample, sizeof(T) * nnz, cudaMemcpyDefault, c.stream));
-                UMAPB_CUDA(cudaMemcpyAsync(ep.enneg0.get(), epoch_of_next_negative_sample, sizeof(T) * nnz, cudaMemcpyDefault, c.stream));
+                copy_async(ep.targets.get(), targets, sizeof(int32_t) * nnz, c.stream);
+                copy_async(ep.eps.get(), epochs_per_sample, sizeof(T) * nnz, c.stream);
+                copy_async(ep.enext0.get(), epoch_of_next_sample, sizeof(T) * nnz, c.stream);
+                copy_async(ep.enneg0.get(), epoch_of_next_negative_sample, sizeof(T) * nnz, c.stream);
             }
             // heads from the row pointers
             std::vector<int64_t> hp(static_cast<size_t>(num_obs) + 1);

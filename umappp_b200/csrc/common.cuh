@@ -114,6 +114,11 @@ void pinned_put(void* p);         // no device work may still write it
 cudaStream_t stream_get(bool high_priority = false);   // non-blocking stream of the current device
 void stream_put(cudaStream_t s);  // s must be idle
 
+// cudaMemcpyAsync with the kinds of memory found out, and large arrays in
+// pageable host memory moved by several threads (host_copy.cu).  As there: a
+// pageable source may be changed on return, a pageable destination is complete.
+void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 // Stream-ordered device allocation from the workspace cache; released on the
 // stream it was allocated on when the owner goes away.
 template <typename T>
@@ -202,7 +207,7 @@ public:
             ptr_ = p;
         } else {
             copy_.allocate(n, s);
-            UMAPB_CUDA(cudaMemcpyAsync(copy_.get(), p, n * sizeof(T), cudaMemcpyHostToDevice, s));
+            copy_async(copy_.get(), p, n * sizeof(T), s);
             ptr_ = copy_.get();
         }
     }
@@ -226,14 +231,14 @@ public:
         } else {
             host_ = p;
             copy_.allocate(n, s);
-            if (load) UMAPB_CUDA(cudaMemcpyAsync(copy_.get(), p, n * sizeof(T), cudaMemcpyHostToDevice, s));
+            if (load) copy_async(copy_.get(), p, n * sizeof(T), s);
             ptr_ = copy_.get();
         }
     }
     T* get() const { return ptr_; }
     bool staged() const { return host_ != nullptr; }
     void finish() {
-        if (host_ && n_) UMAPB_CUDA(cudaMemcpyAsync(host_, ptr_, n_ * sizeof(T), cudaMemcpyDeviceToHost, stream_));
+        if (host_ && n_) copy_async(host_, ptr_, n_ * sizeof(T), stream_);
     }
 
 private:
@@ -247,7 +252,7 @@ private:
 // Copies a device value array of type Src into the caller's array of type Dst.
 inline void copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     if (bytes == 0 || dst == nullptr) return;
-    UMAPB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s));
+    copy_async(dst, src, bytes, s);
 }
 
 // ------------------------------------------------------- device context ---
