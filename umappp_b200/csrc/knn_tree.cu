@@ -203,6 +203,193 @@ __global__ void middle_spread_kernel(const unsigned long long* __restrict__ keys
     }
 }
 
+// ---- segments that fit a block ----
+// A segment of up to SMALL_SEG points is split to its leaves by one block: the
+// levels below are the same splits as those of a segment per launch, but for
+// all of its parts at once and without the host.  (A level of launches, with the
+// splits decided on the host, takes 100 us at least, and 20,000 points without
+// clusters had 22 of them: their search takes 2.8 ms instead of 4.1; 11 levels
+// of 2,048 points here take 0.2 ms.  Segments of 4,096 made the search of
+// 30,011 points 5 % slower than it was with 2,048.)
+constexpr int SMALL_SEG = 2048;
+constexpr int SMALL_THREADS = 512;
+constexpr int SMALL_ITEMS = SMALL_SEG / SMALL_THREADS;
+constexpr int SMALL_PARTS = 160;   // parts of a segment at most
+
+struct SegPart {
+    int32_t start, len, hard_end;
+};
+
+__global__ void __launch_bounds__(SMALL_THREADS)
+    small_tree_kernel(const float* __restrict__ data, int32_t dim, int32_t* __restrict__ perm,
+                      const SegPart* __restrict__ segs, SegPart* __restrict__ parts, int32_t* __restrict__ num_parts) {
+    using Sort = cub::BlockRadixSort<unsigned long long, SMALL_THREADS, SMALL_ITEMS, int32_t>;
+    // between two sorts: the points, in the parts' order, and their projections
+    // as ordered bits (sorted within the parts)
+    __shared__ union {
+        typename Sort::TempStorage sort;
+        struct {
+            int32_t pt[SMALL_SEG];
+            uint32_t key[SMALL_SEG];
+        } item;
+    } tmp;
+    int32_t* const pt = tmp.item.pt;
+    uint32_t* const key = tmp.item.key;
+    __shared__ uint8_t part_of[SMALL_SEG];
+    __shared__ int32_t start[2][SMALL_PARTS + 1];
+    __shared__ uint8_t hard[2][SMALL_PARTS];
+    __shared__ int32_t left[SMALL_PARTS];    // of the part's cut, negative: a hard one, 0: none
+    __shared__ unsigned long long best[SMALL_PARTS];
+    __shared__ int count, splits;
+    const SegPart seg = segs[blockIdx.x];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < seg.len; i += SMALL_THREADS) {
+        pt[i] = perm[seg.start + i];
+        part_of[i] = 0;
+    }
+    if (tid == 0) {
+        start[0][0] = 0;
+        start[0][1] = seg.len;
+        hard[0][0] = seg.hard_end != 0;
+        count = 1;
+    }
+    __syncthreads();
+    const int rounds = (seg.len + SMALL_THREADS - 1) / SMALL_THREADS;
+    int cur = 0;
+    for (int level = 0; level < 64; ++level) {
+        const int np = count;
+        const int32_t* st = start[cur];
+        if (tid == 0) splits = 0;
+        if (tid < np) best[tid] = 0;
+        __syncthreads();
+        auto active = [&](int q) { return st[q + 1] - st[q] > TREE_LEAF; };
+        // the point a of part q: any one, the same on every run
+        auto first_point = [&](int q) {
+            uint32_t z = (static_cast<uint32_t>(seg.start + st[q]) * 0x9E3779B9u) ^ (static_cast<uint32_t>(level) * 0x85EBCA6Bu);
+            z = (z ^ (z >> 15)) * 0x2C1B3C6Du;
+            z ^= z >> 12;
+            return st[q] + static_cast<int>(z % static_cast<uint32_t>(st[q + 1] - st[q]));
+        };
+        for (int r = 0; r < rounds; ++r) {   // a's farthest point of each part
+            const int i = r * SMALL_THREADS + tid;
+            int q = -1;
+            unsigned long long k = 0;
+            if (i < seg.len && active(part_of[i])) {
+                q = part_of[i];
+                const float* x = data + static_cast<size_t>(pt[i]) * dim;
+                const float* xa = data + static_cast<size_t>(pt[first_point(q)]) * dim;
+                float d2 = 0.0f;
+                for (int d = 0; d < dim; ++d) {
+                    const float v = x[d] - xa[d];
+                    d2 = fmaf(v, v, d2);
+                }
+                k = (static_cast<unsigned long long>(__float_as_uint(d2)) << 32) |
+                    static_cast<unsigned long long>(0xffffffffu - static_cast<uint32_t>(i));
+                if (q >= 0) splits = 1;
+            }
+            warp_segment_max(best, q, k);
+        }
+        __syncthreads();
+        if (!splits) break;   // the same for the whole block
+        for (int i = tid; i < seg.len; i += SMALL_THREADS) {   // projections
+            const int q = part_of[i];
+            uint32_t bits = static_cast<uint32_t>(i);   // a finished part keeps its order
+            if (active(q)) {
+                const int b = static_cast<int>(0xffffffffu - static_cast<uint32_t>(best[q] & 0xffffffffu));
+                const float* x = data + static_cast<size_t>(pt[i]) * dim;
+                const float* xa = data + static_cast<size_t>(pt[first_point(q)]) * dim;
+                const float* xb = data + static_cast<size_t>(pt[b]) * dim;
+                float s = 0.0f;
+                for (int d = 0; d < dim; ++d) s = fmaf(x[d], xa[d] - xb[d], s);
+                bits = float_order_bits(s);
+            }
+            key[i] = bits;
+        }
+        __syncthreads();
+        unsigned long long k[SMALL_ITEMS];
+        int32_t v[SMALL_ITEMS];
+#pragma unroll
+        for (int j = 0; j < SMALL_ITEMS; ++j) {
+            const int i = tid * SMALL_ITEMS + j;
+            k[j] = i < seg.len ? static_cast<unsigned long long>(part_of[i]) << 32 | key[i] : ~0ull;
+            v[j] = i < seg.len ? pt[i] : 0;
+        }
+        __syncthreads();
+        Sort(tmp.sort).Sort(k, v, 0, 40);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SMALL_ITEMS; ++j) {
+            const int i = tid * SMALL_ITEMS + j;
+            if (i < seg.len) {
+                key[i] = static_cast<uint32_t>(k[j]);
+                pt[i] = v[j];
+            }
+        }
+        if (tid < np) best[tid] = 0;
+        __syncthreads();
+        for (int r = 0; r < rounds; ++r) {   // the widest gap of each part's window
+            const int i = r * SMALL_THREADS + tid;
+            int q = -1;
+            unsigned long long g = 0;
+            if (i < seg.len && active(part_of[i])) {
+                const int p = part_of[i], len = st[p + 1] - st[p], at = i - st[p];
+                if (at >= gap_window_first(len) && at <= gap_window_last(len)) {
+                    q = p;
+                    g = (static_cast<unsigned long long>(__float_as_uint(
+                             fmaxf(order_bits_float(key[i]) - order_bits_float(key[i - 1]), 0.0f))) << 32) |
+                        static_cast<unsigned long long>(0xffffffffu - static_cast<uint32_t>(at));
+                }
+            }
+            warp_segment_max(best, q, g);
+        }
+        __syncthreads();
+        if (tid < np) {
+            const int len = st[tid + 1] - st[tid];
+            int cut = 0;
+            if (len > TREE_LEAF) {
+                const float gap = __uint_as_float(static_cast<uint32_t>(best[tid] >> 32));
+                const int at = static_cast<int>(0xffffffffu - static_cast<uint32_t>(best[tid] & 0xffffffffu));
+                const float spread = order_bits_float(key[st[tid] + 3 * len / 4]) - order_bits_float(key[st[tid] + max(1, len / 4)]);
+                // (parts are few enough for the lists even if every one were cut)
+                const bool wide = len >= 2 * TREE_LEAF && np <= SMALL_PARTS / 2 && gap > GAP_FACTOR * (spread / (0.5f * len)) &&
+                                  gap > 0.0f && at > 0 && at < len;
+                cut = wide ? -at : ((len + TREE_LEAF - 1) / TREE_LEAF + 1) / 2 * TREE_LEAF;
+            }
+            left[tid] = cut;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            int m = 0;
+            for (int q = 0; q < np; ++q) {
+                start[cur ^ 1][m] = st[q];
+                if (left[q] != 0) {
+                    hard[cur ^ 1][m++] = left[q] < 0;
+                    start[cur ^ 1][m] = st[q] + (left[q] < 0 ? -left[q] : left[q]);
+                }
+                hard[cur ^ 1][m++] = hard[cur][q];
+            }
+            start[cur ^ 1][m] = seg.len;
+            count = m;
+        }
+        __syncthreads();
+        cur ^= 1;
+        for (int i = tid; i < seg.len; i += SMALL_THREADS) {   // the part that holds i: the last that starts at or before it
+            int lo = 0, hi = count - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (start[cur][mid] <= i) lo = mid; else hi = mid - 1;
+            }
+            part_of[i] = static_cast<uint8_t>(lo);
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < seg.len; i += SMALL_THREADS) perm[seg.start + i] = pt[i];
+    for (int q = tid; q < count; q += SMALL_THREADS)
+        parts[static_cast<size_t>(blockIdx.x) * SMALL_PARTS + q] =
+            SegPart{seg.start + start[cur][q], start[cur][q + 1] - start[cur][q], hard[cur][q]};
+    if (tid == 0) num_parts[blockIdx.x] = count;
+}
+
 // row_map[run_dst[r] + i] = perm[run_src[r] + i] for the points of every run.
 __global__ void place_runs_kernel(const int32_t* __restrict__ perm, int32_t nrun, const int32_t* __restrict__ run_src,
                                   const int32_t* __restrict__ run_len, const int32_t* __restrict__ run_dst, int32_t n,
@@ -454,12 +641,9 @@ void knn_tree_order(const float* data, int32_t dim, const std::vector<int32_t>& 
     // two hard cuts, padded to whole tiles); soft cuts keep tile alignment,
     // hard cuts (at a wide gap of the projections, as between two clusters)
     // start a new run, so that no tile spans the gap.
-    struct Seg {
-        int32_t start, len;
-        bool hard_end;
-    };
+    using Seg = SegPart;
     std::vector<Seg> seg(ninst);
-    for (int i = 0; i < ninst; ++i) seg[i] = {inst[i], inst[i + 1] - inst[i], true};
+    for (int i = 0; i < ninst; ++i) seg[i] = {inst[i], inst[i + 1] - inst[i], 1};
     uint64_t h = 0x9E3779B97F4A7C15ull;
     auto next = [&h]() {   // splitmix64: the choice of the direction's first point
         uint64_t z = (h += 0x9E3779B97F4A7C15ull);
@@ -474,7 +658,7 @@ void knn_tree_order(const float* data, int32_t dim, const std::vector<int32_t>& 
         std::vector<int32_t> ast, aoff(1, 0), aa;
         std::vector<int64_t> moff(1, 0);
         for (int g = 0; g < nseg; ++g) {
-            if (seg[g].len <= TREE_LEAF) continue;
+            if (seg[g].len <= SMALL_SEG) continue;   // split by one block below
             ast.push_back(seg[g].start);
             aa.push_back(seg[g].start + static_cast<int32_t>(next() % static_cast<uint64_t>(seg[g].len)));
             aoff.push_back(aoff.back() + seg[g].len);
@@ -541,7 +725,7 @@ void knn_tree_order(const float* data, int32_t dim, const std::vector<int32_t>& 
         int j = 0;
         for (int g = 0; g < nseg; ++g) {
             const Seg x = seg[g];
-            if (x.len <= TREE_LEAF) {
+            if (x.len <= SMALL_SEG) {
                 nseg2.push_back(x);
                 continue;
             }
@@ -551,17 +735,43 @@ void knn_tree_order(const float* data, int32_t dim, const std::vector<int32_t>& 
                               gap[j] > 0.0f;
             if (hard) {
                 const int32_t left = gpos[j];
-                nseg2.push_back({x.start, left, true});
+                nseg2.push_back({x.start, left, 1});
                 nseg2.push_back({x.start + left, x.len - left, x.hard_end});
             } else {
                 const int32_t tiles = (x.len + TREE_LEAF - 1) / TREE_LEAF;
                 const int32_t left = (tiles + 1) / 2 * TREE_LEAF;
-                nseg2.push_back({x.start, left, false});
+                nseg2.push_back({x.start, left, 0});
                 nseg2.push_back({x.start + left, x.len - left, x.hard_end});
             }
             ++j;
         }
         seg.swap(nseg2);
+    }
+    std::vector<Seg> small;
+    for (const Seg& x : seg)
+        if (tree && x.len > TREE_LEAF) small.push_back(x);
+    if (!small.empty()) {
+        DevArray<Seg> d_small(small.size(), s), d_parts(small.size() * SMALL_PARTS, s);
+        DevArray<int32_t> d_num(small.size(), s);
+        UMAPB_CUDA(cudaMemcpyAsync(d_small.get(), small.data(), small.size() * sizeof(Seg), cudaMemcpyHostToDevice, s));
+        small_tree_kernel<<<static_cast<unsigned>(small.size()), SMALL_THREADS, 0, s>>>(data, dim, perm.get(), d_small.get(),
+                                                                                       d_parts.get(), d_num.get());
+        UMAPB_LAUNCH_CHECK();
+        std::vector<Seg> parts(small.size() * SMALL_PARTS), all;
+        std::vector<int32_t> num(small.size());
+        UMAPB_CUDA(cudaMemcpyAsync(parts.data(), d_parts.get(), parts.size() * sizeof(Seg), cudaMemcpyDeviceToHost, s));
+        UMAPB_CUDA(cudaMemcpyAsync(num.data(), d_num.get(), num.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        UMAPB_SYNC(s);
+        size_t b = 0;
+        for (const Seg& x : seg) {
+            if (x.len <= TREE_LEAF) {
+                all.push_back(x);
+                continue;
+            }
+            for (int32_t q = 0; q < num[b]; ++q) all.push_back(parts[b * SMALL_PARTS + q]);
+            ++b;
+        }
+        seg.swap(all);
     }
 
     // runs (segments up to a hard end) laid out one after another, each padded to whole tiles
