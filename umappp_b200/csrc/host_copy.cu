@@ -37,6 +37,7 @@ constexpr int MAX_THREADS = 4;   // the caller among them
 class CopyThreads {
 public:
     std::mutex owner;
+    std::atomic<bool> busy{false};   // set by the owner for a row of jobs: the threads stay awake between them
 
     void copy(char* dst, const char* src, size_t bytes) {
         start();
@@ -88,9 +89,10 @@ private:
     void serve() {
         uint64_t done = 0;   // the last job seen
         while (true) {
-            // a copy is a row of jobs: wait for the next one awake for a while
+            // awake between the jobs of one copy, and shortly after it (a call copies several arrays)
+            int spin = 0;
             uint64_t job = state_.load(std::memory_order_acquire) >> JOB;
-            for (int spin = 0; job == done && spin < 500; ++spin) {
+            while (job == done && (busy.load(std::memory_order_relaxed) || ++spin < 100)) {
                 std::this_thread::yield();
                 job = state_.load(std::memory_order_acquire) >> JOB;
             }
@@ -198,6 +200,10 @@ void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s) {
             Slots* st = lock.owns_lock() ? device_slots() : nullptr;
             if (st) {
                 const double t0 = trace_enabled() ? host_ms() : 0.0;
+                struct Awake {
+                    Awake() { copy_threads().busy.store(true, std::memory_order_relaxed); }
+                    ~Awake() { copy_threads().busy.store(false, std::memory_order_relaxed); }
+                } awake;
                 try {
                     if (up) to_device(*st, static_cast<char*>(dst), static_cast<const char*>(src), bytes, s);
                     else to_host(*st, static_cast<char*>(dst), static_cast<const char*>(src), bytes, s);
