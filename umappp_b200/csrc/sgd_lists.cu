@@ -13,10 +13,12 @@
 // takes the queue 32 edges at a time with all lanes busy -- schedule step,
 // Philox draws, a scan that places every edge's entries (rows start at
 // multiples of LIST_ALIGN), entries staged in shared memory and written out in
-// order.  Bound by instruction issue, about 500 warp instructions per 32
-// firing edges (the scan 85, the samples 130): 0.23 ms an epoch at a million
-// points and 26 million edges, and 0.06 ms to size the lists.  An edge per
-// thread without the queue had 0.28 of the lanes busy in all of it.
+// order.  Bound by instruction issue, about 450 warp instructions per 32
+// firing edges (the samples 130, the two sums that place the entries 35), and
+// by the chains between them: at a million points, 200 epochs take 121 ms with
+// six blocks per SM, 124 with five, 127 with five and one scan that carried
+// the rows' starts along (85 instructions).  An edge per thread without the
+// queue had 0.28 of the lanes busy in all of it.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -30,7 +32,7 @@ namespace {
 
 constexpr int GEN_WARPS = 4;
 // Blocks per SM, alone and beside epochs (which need half of the registers).
-constexpr int GEN_BLOCKS = 5, GEN_BLOCKS_BESIDE = 3;
+constexpr int GEN_BLOCKS = 6, GEN_BLOCKS_BESIDE = 3;
 constexpr int STAGE = 512;   // entries staged per 32 firing edges (they have 6 each on average)
 constexpr int LATE = 32;     // edges with more than 8 samples kept for the end of an epoch
 
@@ -87,6 +89,15 @@ __global__ void segment_rows_kernel(int32_t n, const int64_t* __restrict__ ptr, 
 }
 
 __device__ __forceinline__ uint32_t round_up(uint32_t x) { return (x + (LIST_ALIGN - 1)) & ~uint32_t(LIST_ALIGN - 1); }
+
+// Inclusive sum over the lanes of a warp.
+__device__ __forceinline__ uint32_t prefix_sum(uint32_t x) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)   // the shuffle's predicate: a lane with a source
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .u32 r;\n\t"
+                     "shfl.sync.up.b32 r|p, %0, %1, 0, 0xffffffff;\n\t@p add.u32 %0, %0, r;\n\t}" : "+r"(x) : "r"(o));
+    return x;
+}
 
 // Observation range of the instance that owns row h.
 __device__ __forceinline__ void instance_range(int32_t h, const ListStream& p, int32_t& base, uint32_t& size) {
@@ -240,22 +251,16 @@ __global__ void __launch_bounds__(GEN_WARPS * 32, GEN_BLOCKS) schedule_kernel(co
                     int32_t prev = __shfl_up_sync(0xffffffffu, h, 1);
                     if (lane == 0) prev = last;
                     // Placing 32 edges after one another, rows at multiples of
-                    // LIST_ALIGN: edges 0..lane take the position p to p + a, or,
-                    // when a row starts among them, to round_up(p + a) + b.
+                    // LIST_ALIGN: a row starts where the one before it ends, which
+                    // started at such a multiple too (or before this group, whose
+                    // position is known), so its padding follows from the plain sums.
                     const bool opens = on && h != prev;
-                    uint32_t a = opens ? 0u : cnt, b = opens ? cnt : 0u, f = opens;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        uint32_t fl = __shfl_up_sync(0xffffffffu, f, o);
-                        const uint32_t al = __shfl_up_sync(0xffffffffu, a, o), bl = __shfl_up_sync(0xffffffffu, b, o);
-                        fl = lane >= o ? fl : 0;
-                        const uint32_t sum_a = lane >= o ? al + a : a;   // no row starts to the left
-                        b = fl ? (f ? round_up(bl + a) + b : bl + a) : b;
-                        a = fl ? al : sum_a;
-                        f |= fl;
-                    }
-                    const uint32_t end = f ? round_up(pos + a) + b : pos + a;
-                    const uint32_t off = end - cnt;
+                    const uint32_t ahead = prefix_sum(cnt) - cnt;
+                    const unsigned opened = __ballot_sync(0xffffffffu, opens) & below;
+                    const uint32_t at_open = __shfl_sync(0xffffffffu, ahead, opened ? 31 - __clz(opened) : 0);
+                    const uint32_t pad = opens ? ((opened ? at_open : 0u - pos) - ahead) & (LIST_ALIGN - 1) : 0u;
+                    const uint32_t off = pos + ahead + prefix_sum(pad);
+                    const uint32_t end = off + cnt;
                     const int32_t next = __shfl_down_sync(0xffffffffu, h, 1);
                     const bool ends = on && (lane == 31 || next != h);
                     ListSpan* sp = spans + h;
