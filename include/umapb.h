@@ -409,9 +409,8 @@ int umapb_optimize_layout(int dtype, size_t num_dim, void* embedding, int32_t nu
  * its own instance only), one similarity / union / schedule pass over the
  * block-diagonal graph (each instance keeps its own maximum weight), and one
  * SGD launch per epoch over all instances (negative samples drawn inside the
- * head's instance), the epochs recorded as one CUDA graph, with the launch
- * shape chosen by the autotuner.  All instances must resolve to the same
- * epoch count (set opt->num_epochs when their sizes differ across 10000).
+ * head's instance).  All instances must resolve to the same epoch count (set
+ * opt->num_epochs when their sizes differ across 10000).
  * stage_ms (may be NULL) receives the 7 stage times of umapb_status_stage_ms.
  */
 int umapb_batch_run(int dtype, int32_t num_instances, const int32_t* sizes, size_t data_dim, const void* data,

@@ -66,6 +66,37 @@ def test_long_rows_match_serial(umap, monkeypatch, edges, num_dim, window_bytes)
     assert np.array_equal(dev.epoch_of_next_negative_sample, ep.enneg)
 
 
+def stars(n, heads, num_dim, dtype, seed=5):
+    """n points of which the first 'heads' have edges, up to 90 each (every fifth none), to tails that no other has."""
+    rng = np.random.default_rng(seed)
+    count = np.zeros(n, dtype=np.int64)
+    count[:heads] = np.where(np.arange(heads) % 5 == 4, 0, rng.integers(1, 91, size=heads))
+    assert heads + count.sum() <= n
+    w = rng.uniform(0.02, 1.0, size=count.sum()).astype(dtype)
+    g = oracle.CSR(np.concatenate([[0], np.cumsum(count)]), (heads + np.arange(count.sum())).astype(np.int32), w)
+    return oracle.similarities_to_epochs(g, 40, 5.0), rng.normal(scale=3.0, size=(n, num_dim)).astype(dtype)
+
+
+# 49,152 points have 6,144 rows in flight, the most that relays take; 49,160 are taken by single warps
+@pytest.mark.parametrize("n,heads", [(900, 9), (12000, 250), (49152, 700), (49160, 700)])
+@pytest.mark.parametrize("num_dim,dtype", [(1, np.float32), (2, np.float32), (3, np.float32), (7, np.float32),
+                                           (1, np.float64), (2, np.float64), (3, np.float64), (40, np.float64)])
+def test_separate_rows_match_serial(umap, n, heads, num_dim, dtype):
+    """Rows without common points and no repulsion: the serial run's layout, to TOL in FP64.  In FP32 a step's
+    gradient is off by 2^-19 of at most 4 (the approximate logarithm, power and reciprocal and four products), a
+    position by half a unit (at most 2^-20 below 32), and a row's head takes at most 90 steps an epoch at rates that
+    add up to 2.05; four times their sum, as early errors may grow where a step overshoots."""
+    ep, Y = stars(n, heads, num_dim, dtype)
+    dev = device_epochs(umap, ep)
+    Yd = Y.copy()
+    umap.optimize_layout(num_dim, Yd, dev, 1.577, 0.895, 0.0, 0.1, 99, 40, 5.0)
+    start = Y.copy()
+    oracle.optimize_layout(num_dim, Y, ep, 1.577, 0.895, 0.0, 0.1, 99, 40)
+    tol = TOL * np.abs(Y).max() if dtype == np.float64 else 4 * (90 * 2.05 * 4 * 2.0 ** -19 + 90 * 40 * 2.0 ** -20)
+    assert np.max(np.abs(Y - start)) > 10 * tol
+    assert np.max(np.abs(Yd - Y)) <= tol
+
+
 @pytest.mark.parametrize("num_dim", [2, 3, 4])
 def test_unaligned_layout(umap, num_dim):
     torch = pytest.importorskip("torch")

@@ -4,21 +4,23 @@
 // firing edges in CSR order: an attractive step that moves head and tail,
 // then that edge's negative samples, which move the head only.  Here one
 // thread (or a group of lanes, for layouts of more than four dimensions) takes
-// one head's whole row in that order, from a flat list of the points the head
+// the steps of one head's whole row in that order, from a flat list of the points the head
 // meets in this epoch, which sgd_lists.cu has worked out ahead for a window of
 // epochs: the schedule and the samples do not depend on the layout.  What is
 // left is the chain that does: gather a point, take its step, move the head.
 //
 // Concurrency.  All rows of an epoch run at once (one launch per epoch), in a
 // claim order fixed per epoch (epoch_order_kernel): chunks of rows of
-// neighbouring index, rows that would end last ahead of them.  A row's head is kept in registers and
-// its displacement is added to the embedding (vector atomic add) after every
-// firing edge; tails move by vector atomic adds.  Measured on a
+// neighbouring index, rows that would end last ahead of them.  A row's head is
+// kept in registers and its displacement is added to the embedding (vector
+// atomic add) after every firing edge, or every eight entries (the relay
+// kernel); tails move by vector atomic adds.  Measured on a
 // 1,000,000-point mixture against the serial reference's edge cross-entropy:
 // splitting a hub's row into concurrently processed pieces, or publishing the
 // head's move only at the end of a long row, leaves the layout about 1-1.5 %
 // tighter than the reference's; whole rows with the head published after each
-// firing edge come within about 0.3 %.
+// firing edge come within about 0.3 %, and so do the relays' at 5,000 and 40,000
+// points.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -384,11 +386,45 @@ struct ListHead {
     }
 };
 
+// One entry's step: moves head by its gradient at y (times rate); pull is the
+// opposite move, the target's where the entry is one.
+template <bool FIXED, typename T, int NC, int G>
+__device__ __forceinline__ void take_step(Point<T, NC, G>& head, const Point<T, NC, G>& y, bool attract, T rate,
+                                          const StepParams<T>& p, Point<T, NC, G>& pull) {
+    T diff[NC], d2 = 0, grad[NC];
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+        diff[j] = head.v[j] - y.v[j];
+        d2 = FIXED ? d2 + diff[j] * diff[j] : madd(d2, diff[j], diff[j]);
+    }
+    if constexpr (G > 1) {   // the group's lanes share the row
+        const unsigned group = (G == 32 ? 0xffffffffu : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) d2 += __shfl_xor_sync(group, d2, o, G);
+    }
+    d2 = floor_eps(d2);
+    if constexpr (FIXED) {
+        const T cf = transform_coef(d2, attract, p);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) grad[j] = cf * diff[j];
+    } else {
+        step_gradient(d2, attract, diff, p, grad);
+    }
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+        const T g = clamp4(grad[j]);
+        head.v[j] = FIXED ? head.v[j] + rate * g : madd(head.v[j], rate, g);
+        pull.v[j] = -(rate * g);
+    }
+}
+
 // One row's list applied to its head, CH entries at a time: while CH steps
 // run, the points of the next CH are gathered and the entries after those
 // read.  The head's move is published at every firing edge, together with the
 // edge's own pull on its tail, and a long row's head re-read after every 256
-// entries, with the other rows' pulls on it.  (Published after every 8 entries
+// entries, with the other rows' pulls on it.  (Pulls kept in shared memory and
+// added at a chunk's end, the head's move once a chunk: 25.7 ms against 21.9
+// for a batch of 91,000 points, 177 against 170 for a million.)  (Published after every 8 entries
 // instead, a step costs 151 cycles against 200, but the layout's cross-entropy
 // at 100,000 points is 2.9 % above the reference's; as it is, 0.05 %.)
 // What bounds a row is the chain of its steps -- some 100 cycles each of
@@ -438,34 +474,9 @@ struct RowWalk {
         }
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
-            const bool attract = e.e[i] < 0;
-            T diff[NC], d2 = 0, grad[NC];
-#pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                diff[j] = head.v[j] - y[i].v[j];
-                d2 = FIXED ? d2 + diff[j] * diff[j] : madd(d2, diff[j], diff[j]);
-            }
-            if constexpr (G > 1) {   // the group's lanes share the row
-                const unsigned group = (G == 32 ? 0xffffffffu : (1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
-#pragma unroll
-                for (int o = G / 2; o > 0; o >>= 1) d2 += __shfl_xor_sync(group, d2, o, G);
-            }
-            d2 = floor_eps(d2);
-            if constexpr (FIXED) {
-                const T cf = transform_coef(d2, attract, p);
-#pragma unroll
-                for (int j = 0; j < NC; ++j) grad[j] = cf * diff[j];
-            } else {
-                step_gradient(d2, attract, diff, p, grad);
-            }
             const T rate = (FIXED ? c * CH + i < l.cnt : e.e[i] != h) ? p.alpha : T(0);
             Point<T, NC, G> pull;
-#pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                const T g = clamp4(grad[j]);
-                head.v[j] = FIXED ? head.v[j] + rate * g : madd(head.v[j], rate, g);
-                pull.v[j] = -(rate * g);
-            }
+            take_step<FIXED>(head, y[i], e.e[i] < 0, rate, p, pull);
             if (!FIXED) {
                 pull.add_if_negative(e.e[i], Y, e.point(i), dim);
                 publish(e.e[i]);
@@ -529,6 +540,335 @@ __global__ void __launch_bounds__(ROW_BLOCK, ROW_BLOCKS)
         if (!more) break;
         cur = nxt;
         head_of_list.load(list, cur.start8, cur.count);
+    }
+}
+
+// ------------------------------------------ few rows in flight: the relay --
+// Three warps work on the same rows ('share' of them, at most 32 / G), a chunk
+// of CH entries of each at a time.  The first (fetch_rows) claims the rows in
+// the epoch's order, reads their lists, gathers the points and leaves them in
+// shared memory; the second (walk_chunk) takes the steps and does nothing
+// else; the third (publish_rows) adds a chunk's moves to the embedding: every
+// firing edge's pull on its tail, and the head's move.
+// With few rows in flight an epoch takes as long as its longest row's chain of
+// steps.  The dependent arithmetic of a step is 111 cycles (2-d float); in a
+// warp that gathers and adds by itself it takes 205 with one row and 258 with
+// 32, as a lone warp issues an instruction every 4-5 cycles and each add to
+// global memory holds it up for some 40, active lanes or none.  Here it takes
+// 142 with up to 8 rows, 227 with 32.  Where the SMs are full the three warps'
+// instructions cost more than the chain (relay_rows()).
+// About every RELOAD entries a head takes over the other rows' pulls on it.
+constexpr int RELAY_WARPS = 3;
+constexpr uint32_t RELOAD = 256;
+// READY: points are there (fetching -> walking warp); DONE: steps are done
+// (walking -> fetching and publishing warp).  Each for two buffers.
+// START: the first chunk's kind is there, for the publishing warp.
+enum RowBarrier { READY = 1, DONE = 3, START = 5 };
+
+template <int ID, int WARPS>
+__device__ __forceinline__ void row_sync() {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(32 * WARPS) : "memory");
+}
+template <int ID, int WARPS>
+__device__ __forceinline__ void row_arrive() {
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(32 * WARPS) : "memory");
+}
+
+// What the warps hand one another.  Chunk s has its points in buffer s % 2,
+// which is filled again once the steps are done, and its moves in set s % 4,
+// which chunk s + 4 uses: it is fetched after DONE of chunk s + 2, where the
+// publishing warp arrives when it is done with chunk s + 1.
+// A MEASURE chunk's publication finds out what others have added to the heads;
+// the SHIFT chunk, three later, takes it over.
+enum ChunkKind { CHUNK_NEXT, CHUNK_FIRST, CHUNK_MEASURE, CHUNK_SHIFT, CHUNK_STOP };
+template <typename T, int NC, int CH>
+struct RowMail {
+    // a point or move with its entry: one access where they fit one
+    static constexpr bool packed = NC * sizeof(T) < 16;
+    struct alignas(NC * sizeof(T) > 4 ? 16 : 8) Packed {
+        T v[NC];
+        int32_t e;
+    };
+    struct alignas(16) Vector {
+        T v[NC];
+    };
+    struct Split {
+        Vector at[CH][32];
+        int32_t e[CH][32];
+    };
+    struct Joint {
+        Packed at[CH][32];
+    };
+    using Items = typename std::conditional<packed, Joint, Split>::type;
+    template <int G>
+    static __device__ __forceinline__ void put(Items& m, int i, int lane, const Point<T, NC, G>& y, int32_t e) {
+        if constexpr (packed) {
+            Packed q;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) q.v[j] = y.v[j];
+            q.e = e;
+            m.at[i][lane] = q;
+        } else {
+            Vector q;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) q.v[j] = y.v[j];
+            m.at[i][lane] = q;
+            m.e[i][lane] = e;
+        }
+    }
+    template <int G>
+    static __device__ __forceinline__ int32_t get(const Items& m, int i, int lane, Point<T, NC, G>& y) {
+        const auto q = m.at[i][lane];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) y.v[j] = q.v[j];
+        if constexpr (packed) return q.e;
+        else return m.e[i][lane];
+    }
+    struct Place {
+        T v[NC];
+    };
+    Items point[2];          // the entries' points
+    Items pull[2][2];        // [s / 2 % 2][s % 2] from here on: the pulls at firing edges, and their tails
+    Place last[2][2][32];    // where the heads are in the end
+    Place start[2][2][32];   // where they are first (CHUNK_FIRST)
+    int32_t row[2][2][32];
+    uint32_t edges[2][2][32];   // which entries are firing edges; bit 31: the row has entries here
+    int kind[2][2];
+    Place shift[32];         // what the heads take over
+};
+
+// One chunk's steps; false: there are no more.
+template <int B, typename T, int NC, int G, int CH>
+__device__ __forceinline__ bool walk_chunk(RowMail<T, NC, CH>& m, int half, Point<T, NC, G>& head, int32_t& h,
+                                           const StepParams<T>& p, int lane) {
+    row_sync<READY + B, 2>();
+    const int kind = m.kind[half][B];
+    if (kind == CHUNK_STOP) return false;
+    if (kind == CHUNK_FIRST) {
+        h = m.row[half][B][lane];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) head.v[j] = m.start[half][B][lane].v[j];
+    } else if (kind == CHUNK_SHIFT) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) head.v[j] += m.shift[lane].v[j];
+    }
+    Point<T, NC, G> y[CH];
+    int32_t e[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) e[i] = RowMail<T, NC, CH>::get(m.point[B], i, lane, y[i]);
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+        Point<T, NC, G> pull;
+        take_step<false>(head, y[i], e[i] < 0, e[i] != h ? p.alpha : T(0), p, pull);
+        if (e[i] < 0) RowMail<T, NC, CH>::put(m.pull[half][B], i, lane, pull, e[i] & INT32_MAX);
+    }
+#pragma unroll
+    for (int j = 0; j < NC; ++j) m.last[half][B][lane].v[j] = head.v[j];
+    row_arrive<DONE + B, 3>();
+    return true;
+}
+
+// The fetching warp's way along the lists of its rows, chunk by chunk.  Rows are
+// claimed when the lists at hand are about to end, not earlier: a claimed row
+// waits for the longest one before it.
+template <typename T, int NC, int G, int CH>
+struct RowCursor {
+    const RowTask* __restrict__ tasks;
+    const int32_t nrows;
+    const int32_t* __restrict__ lists;
+    int* __restrict__ counter;
+    const int share;   // rows claimed at a time
+    const int lane;
+    // of the chunk last read
+    Entries<CH> e;
+    int32_t h = 0;
+    bool on = false;          // the row has entries here
+    int kind = CHUNK_FIRST;
+    // of the rows at hand, and the next claim
+    const int32_t* list = nullptr;
+    uint32_t c = 0, chunks = 0, most = 0;
+    int32_t base = 0;
+    int4 task = make_int4(0, 0, 0, 0);
+    bool claimed = false, fetched = false;
+
+    __device__ __forceinline__ void claim() {
+        if (lane == 0) base = atomicAdd(counter, share);
+        claimed = true;
+    }
+    __device__ __forceinline__ void fetch() {
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const int32_t i = base + lane / G;
+        task = lane / G < share && i < nrows ? __ldg(reinterpret_cast<const int4*>(tasks) + i) : make_int4(0, 0, 0, 0);
+        fetched = true;
+    }
+    __device__ __forceinline__ void read() {
+        const uint32_t phase = c % (RELOAD / CH);
+        kind = c < RELOAD / CH || (phase != 0 && phase != 3) ? CHUNK_NEXT : phase == 0 ? CHUNK_MEASURE : CHUNK_SHIFT;
+        while (c >= most) {
+            if (!claimed) claim();
+            if (!fetched) fetch();
+            if (base >= nrows) {
+                kind = CHUNK_STOP;
+                on = false;
+                return;
+            }
+            h = task.x;
+            list = lists + static_cast<int64_t>(static_cast<uint32_t>(task.y)) * LIST_ALIGN;
+            chunks = (static_cast<uint32_t>(task.z) + CH - 1) / CH;
+            most = __reduce_max_sync(0xffffffffu, chunks);
+            c = 0;
+            claimed = fetched = false;
+            kind = CHUNK_FIRST;
+        }
+        if (claimed && !fetched) fetch();
+        if (c + 3 >= most && !claimed) claim();
+        on = c < chunks;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) e.e[i] = h;
+        if (on) e.load(list + c * CH);
+        ++c;
+    }
+};
+
+template <typename T, int NC, int G, int CH>
+__device__ __forceinline__ void fetch_rows(RowMail<T, NC, CH>& m, const RowTask* __restrict__ tasks, int32_t nrows,
+                                           const int32_t* __restrict__ lists, const T* __restrict__ Y, int dim,
+                                           int* __restrict__ counter, int share, int lane) {
+    RowCursor<T, NC, G, CH> ahead{tasks, nrows, lists, counter, share, lane};
+    // the chunk whose points are being gathered
+    Entries<CH> e;
+    int32_t h;
+    bool on;
+    int kind;
+    Point<T, NC, G> y[CH], head;
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) y[i].v[j] = head.v[j] = T(0);
+    auto gather = [&] {
+        e = ahead.e, h = ahead.h, on = ahead.on, kind = ahead.kind;
+        if (kind == CHUNK_STOP) return;
+        if (on) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) y[i].load(Y, e.point(i), dim);
+        }
+        if (kind == CHUNK_FIRST) head.load(Y, h, dim);
+        ahead.read();
+    };
+    int filled[2];   // the chunks' kinds
+    auto fill = [&](int half, auto buffer) {
+        constexpr int B = decltype(buffer)::value;
+        filled[B] = kind;
+        if (lane == 0) m.kind[half][B] = kind;
+        if (kind != CHUNK_STOP) {
+            uint32_t fires = on ? 1u << 31 : 0u;
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                RowMail<T, NC, CH>::put(m.point[B], i, lane, y[i], e.e[i]);
+                fires |= (static_cast<uint32_t>(e.e[i]) >> 31) << i;
+            }
+            m.edges[half][B][lane] = fires;
+            if (kind == CHUNK_FIRST) {
+                m.row[half][B][lane] = h;
+#pragma unroll
+                for (int j = 0; j < NC; ++j) m.start[half][B][lane].v[j] = head.v[j];
+            }
+        }
+        row_arrive<READY + B, 2>();
+    };
+    using Zero = std::integral_constant<int, 0>;
+    using One = std::integral_constant<int, 1>;
+    // Once the steps of buffer B's chunk are done it is filled again, and the
+    // points of the chunk after that are gathered.  False: the chunks end.
+    int half = 0;
+    auto turn = [&](auto buffer) {
+        constexpr int B = decltype(buffer)::value;
+        row_sync<DONE + B, 3>();
+        if (filled[1 - B] == CHUNK_STOP) return false;
+        fill(half ^ 1, buffer);
+        if (kind != CHUNK_STOP) gather();
+        return true;
+    };
+    ahead.read();
+    gather();
+    fill(0, Zero());
+    row_arrive<START, 2>();
+    if (kind == CHUNK_STOP) return;
+    gather();
+    fill(0, One());
+    if (kind != CHUNK_STOP) gather();
+    for (; turn(Zero()) && turn(One()); half ^= 1) {
+    }
+}
+
+// Adds one chunk's moves; false: there are no more.
+template <int B, typename T, int NC, int G, int CH>
+__device__ __forceinline__ bool publish_chunk(RowMail<T, NC, CH>& m, int half, Point<T, NC, G>& pub, int32_t& h,
+                                              T* __restrict__ Y, int dim, int lane) {
+    const int kind = m.kind[half][B];   // written before DONE of the chunk before (or START)
+    if (kind == CHUNK_STOP) return false;
+    row_sync<DONE + B, 3>();
+    if (kind == CHUNK_FIRST) {
+        h = m.row[half][B][lane];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) pub.v[j] = m.start[half][B][lane].v[j];
+    } else if (kind == CHUNK_SHIFT) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) pub.v[j] += m.shift[lane].v[j];
+    }
+    const uint32_t edges = m.edges[half][B][lane];
+    const bool on = edges >> 31;
+    uint32_t left = edges & 0x7fffffffu;
+    while (__any_sync(0xffffffffu, left)) {   // each lane's next firing edge
+        Point<T, NC, G> pull;
+        const int32_t tail = RowMail<T, NC, CH>::get(m.pull[half][B], left ? __ffs(left) - 1 : 0, lane, pull);
+        pull.add_if_negative(left ? -1 : 0, Y, tail, dim);
+        left &= left - 1;
+    }
+    Point<T, NC, G> move;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+        const T at = m.last[half][B][lane].v[j];
+        move.v[j] = at - pub.v[j];
+        pub.v[j] = at;
+    }
+    move.add_if_negative(on ? -1 : 0, Y, h, dim);
+    if (kind == CHUNK_MEASURE) {   // what is there beyond what was added from here
+        Point<T, NC, G> now;
+        if (on) now.reload(Y, h, dim);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) m.shift[lane].v[j] = on ? now.v[j] - pub.v[j] : T(0);
+    }
+    return true;
+}
+
+// One epoch by relays.
+template <typename T, int NC, int G, int CH>
+__global__ void __launch_bounds__(32 * RELAY_WARPS, NC == 1 || G == 1 && NC * sizeof(T) < 16 ? 8 : 6)
+    sgd_relay_kernel(const RowTask* __restrict__ tasks, int32_t nrows, const int32_t* __restrict__ list,
+                    T* __restrict__ Y, int dim, int* __restrict__ counter, int share, const StepParams<T> p) {
+    __shared__ RowMail<T, NC, CH> mail;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        fetch_rows<T, NC, G, CH>(mail, tasks, nrows, list, Y, dim, counter, share, lane);
+        return;
+    }
+    Point<T, NC, G> head;
+    int32_t h = 0;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) head.v[j] = T(0);
+    if (warp == 1) {
+        for (int half = 0; walk_chunk<0>(mail, half, head, h, p, lane) && walk_chunk<1>(mail, half, head, h, p, lane);
+             half ^= 1) {
+        }
+        return;
+    }
+    row_sync<START, 2>();
+    for (int half = 0; publish_chunk<0>(mail, half, head, h, Y, dim, lane) &&
+                       publish_chunk<1>(mail, half, head, h, Y, dim, lane);
+         half ^= 1) {
     }
 }
 
@@ -661,20 +1001,35 @@ int64_t rows_in_flight(int32_t n, int window_div) {
     return std::min(most, (w + 255) / 256 * 256);
 }
 
-// Blocks of the epoch kernel that are resident at once on the device.
-template <typename T, int NC, int G, int CH>
-int64_t resident_blocks() {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int r = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, sgd_rows_kernel<T, NC, G, CH>, ROW_BLOCK, 0) != cudaSuccess ||
-            r < 1) {
-            cudaGetLastError();
-            r = 1;
-        }
-        per_sm = r;
+// Blocks of an epoch kernel that are resident at once on the device.
+template <class K>
+int64_t resident_blocks(K kernel, int threads) {
+    int r = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kernel, threads, 0) != cudaSuccess || r < 1) {
+        cudaGetLastError();
+        r = 1;
     }
-    return static_cast<int64_t>(per_sm) * sm_count();
+    return static_cast<int64_t>(r) * sm_count();
+}
+
+// Whether an epoch with this many rows in flight is run by relays: as long as
+// its time is the longest rows' chains rather than what the SMs issue.  100
+// epochs (whole runs, relays / single warps, 15 neighbours): 1,000 x 2 f32
+// points 3.6 / 4.7 ms, 10,000 7.8 / 10.2, 45,000 (5,632 rows in flight) 13.0 /
+// 14.8, 64,000 (8,192) 15.5 / 15.5, a batch of 91,000 (11,520) 15.9 / 13.4;
+// 30,000 x 5 f32 13.8 / 21.1, 20,000 x 2 f64 31.7 / 39.4.
+bool relay_rows(int64_t rows) { return rows <= 6144; }
+
+// Rows per relay: the fewest with which RELAY_BLOCKS per SM hold all rows (a
+// relay's steps are faster with few rows, and it waits for the longest of
+// them).  10,007 x 2 points, 500 epochs: 42.8 ms with 2, 43.7 with 4, 45.7 with
+// 16, and 45.2 with 1, when there are more relays than run at once.
+constexpr int RELAY_BLOCKS = 5;
+template <int G>
+int relay_share(int64_t rows) {
+    int share = 1;
+    while (share < 32 / G && rows > int64_t(RELAY_BLOCKS) * sm_count() * share) share *= 2;
+    return share;
 }
 
 template <typename T>
@@ -844,10 +1199,19 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
                 p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(epoch_t / static_cast<T>(total))));
                 for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
                     constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
-                    const int64_t blocks = std::min((rows * G + ROW_BLOCK - 1) / ROW_BLOCK, resident_blocks<T, NC, G, CH>());
-                    sgd_rows_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), ROW_BLOCK, 0, es>>>(
-                        tasks_[buffer].get() + static_cast<size_t>(e - e0) * n, n, lists_.list(buffer), Yp, stride,
-                        counters.get() + (e - first), p);
+                    const RowTask* tasks = tasks_[buffer].get() + static_cast<size_t>(e - e0) * n;
+                    if (relay_rows(rows)) {
+                        static const int64_t resident = resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS);
+                        const int share = relay_share<G>(rows);
+                        const int64_t blocks = std::min((rows + share - 1) / share, resident);
+                        sgd_relay_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), 32 * RELAY_WARPS, 0, es>>>(
+                            tasks, n, lists_.list(buffer), Yp, stride, counters.get() + (e - first), share, p);
+                    } else {
+                        static const int64_t resident = resident_blocks(sgd_rows_kernel<T, NC, G, CH>, ROW_BLOCK);
+                        const int64_t blocks = std::min((rows * G + ROW_BLOCK - 1) / ROW_BLOCK, resident);
+                        sgd_rows_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), ROW_BLOCK, 0, es>>>(
+                            tasks, n, lists_.list(buffer), Yp, stride, counters.get() + (e - first), p);
+                    }
                 });
                 UMAPB_LAUNCH_CHECK();
             }
