@@ -91,7 +91,8 @@ def l2_random_access_peaks(U) -> dict:
 
 def sgd_roofline(nnz: int, epochs: int, firing: float, negs: float, sgd_ms: float, peaks: dict, l2: dict,
                  traffic, traffic_src) -> dict:
-    """Roofline of the SGD epochs (one launch of sgd_rows_2d_f32 per epoch).
+    """Roofline of the SGD epochs (one launch of sgd_rows_kernel per epoch, over
+    interaction lists that schedule_kernel builds ahead of them; the stage time has both).
     Against HBM: the algorithmic bytes of the schedule and the layout,
     4 nnz + 56 F + 8 N_neg per epoch (F firing edges, N_neg negative samples,
     exact counts from the schedule), over the SGD stage's CUDA-event time,
@@ -107,7 +108,7 @@ def sgd_roofline(nnz: int, epochs: int, firing: float, negs: float, sgd_ms: floa
     sgd_gbs = sgd_bytes / sgd_s / 1e9
     loads, adds = 2.0 * firing + negs, 2.0 * firing
     l2_floor_s = loads / l2["gather_per_s"] + adds / l2["atomic_add_per_s"]
-    return {"bound": "hbm", "kernel": "sgd_rows_2d_f32",
+    return {"bound": "hbm", "kernel": "sgd_rows_kernel",
             "achieved": round(sgd_gbs, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": round(sgd_gbs / peaks["hbm_gbs"], 4), "peak_source": peaks["source"],
             "traffic": traffic, "traffic_unit": "DRAM bytes per epoch launch", "traffic_source": traffic_src,
@@ -282,7 +283,7 @@ def run_ours(args, rank: int, world: int) -> dict | None:
 
     peaks = load_peaks()
     l2 = l2_random_access_peaks(U)
-    traffic_sgd, traffic_sgd_src = load_traffic(args.config, "sgd_rows_2d_f32")
+    traffic_sgd, traffic_sgd_src = load_traffic(args.config, "sgd_rows_kernel")
     roof_sgd = sgd_roofline(nnz, epochs, firing, negs, sgd_ms, peaks, l2, traffic_sgd, traffic_sgd_src)
     # kNN roofline: the distances the pruned search computes (128 x 128 per tile pair,
     # 2*dim FLOP each, the FP32 GEMM count) over the kernel's device time

@@ -422,11 +422,10 @@ __device__ __forceinline__ void take_step(Point<T, NC, G>& head, const Point<T, 
 // run, the points of the next CH are gathered and the entries after those
 // read.  The head's move is published at every firing edge, together with the
 // edge's own pull on its tail, and a long row's head re-read after every 256
-// entries, with the other rows' pulls on it.  (Pulls kept in shared memory and
-// added at a chunk's end, the head's move once a chunk: 25.7 ms against 21.9
-// for a batch of 91,000 points, 177 against 170 for a million.)  (Published after every 8 entries
-// instead, a step costs 151 cycles against 200, but the layout's cross-entropy
-// at 100,000 points is 2.9 % above the reference's; as it is, 0.05 %.)
+// entries, with the other rows' pulls on it.  (The head's move
+// published once per 8 entries: 24.2 ms against 22.0 for a batch of 91,000
+// points, 173.5 against 170.5 for a million; with the pulls kept in shared
+// memory and added then, too: 25.7 and 177.)
 // What bounds a row is the chain of its steps -- some 100 cycles each of
 // dependent arithmetic -- so the steps are straight code of few instructions:
 // the lists are padded with the head itself, and an entry equal to the head
