@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "list_stage.cuh"
 #include "neg_stream.cuh"
 #include "stages.cuh"
 
@@ -34,7 +35,7 @@ constexpr int GEN_WARPS = 4;
 // Blocks per SM, alone and beside epochs (which need half of the registers).
 constexpr int GEN_BLOCKS = 6, GEN_BLOCKS_BESIDE = 3;
 constexpr int STAGE = 512;   // entries staged per 32 firing edges (they have 6 each on average)
-constexpr int LATE = 32;     // edges with more than 8 samples kept for the end of an epoch
+constexpr int LATE = 32;     // edges with more than STAGE_SAMPLES samples kept for the end of an epoch
 
 // Edges of a segment's state kept in shared memory (9 KB per warp either way).
 template <typename T>
@@ -46,7 +47,7 @@ constexpr int seg_target() { return seg_edges<T>() * 3 / 4; }
 template <typename T>
 struct alignas(16) GenWarp {
     T en[seg_edges<T>()], enn[seg_edges<T>()], ep[seg_edges<T>()], epns[seg_edges<T>()];
-    int32_t stage[STAGE + 16];
+    int32_t stage[STAGE];
     uint16_t queue[seg_edges<T>()];
     uint32_t late_off[LATE], late_draws[LATE];
     uint16_t late_edge[LATE];
@@ -223,7 +224,10 @@ __global__ void __launch_bounds__(GEN_WARPS * 32, GEN_BLOCKS) schedule_kernel(co
                 // the stage holds the entries from 'origin', a multiple of LIST_ALIGN, on
                 uint32_t origin = pos & ~uint32_t(LIST_ALIGN - 1);
                 int nlate = 0;
-                if (FILL && pos != origin && lane < LIST_ALIGN) w.stage[lane] = g.list[ebase + origin + lane];   // a row of several chunks
+                if (FILL && pos != origin) {   // a row of several chunks
+                    if (lane < LIST_ALIGN) w.stage[lane] = g.list[ebase + origin + lane];
+                    __syncwarp();
+                }
                 int32_t last = FILL ? __shfl_sync(0xffffffffu, head_of, e) : 0;
                 const uint32_t epoch = static_cast<uint32_t>(g.first + e);
                 ListSpan* spans = FILL ? g.span + static_cast<int64_t>(e) * g.nrows : nullptr;
@@ -277,40 +281,29 @@ __global__ void __launch_bounds__(GEN_WARPS * 32, GEN_BLOCKS) schedule_kernel(co
                     bool again = false;
                     int32_t* out;
                     if (staged) {
-                        // Eight samples are drawn and stored by every lane, whatever it
-                        // needs, from the last to the first and then the target: what a
-                        // lane stores too much (its head, as padding) lies where later
-                        // lanes store with a smaller index, that is, afterwards.  Lanes
-                        // without an edge store behind the stage.
-                        out = w.stage + (on ? off - origin : STAGE);
-                        volatile int32_t* to = out;
-                        if (ends) {   // the row's padding (the next 32 edges overwrite it where they continue the row)
-#pragma unroll
-                            for (int i = 0; i < LIST_ALIGN - 1; ++i) to[cnt + i] = h;
-                        }
+                        out = w.stage + (off - origin);   // (without an edge: nothing is stored)
                         uint32_t low = 0xffffffffu;
-                        int32_t k[8];
+                        int32_t k[STAGE_SAMPLES];
 #pragma unroll
-                        for (int q = 0; q < 8; q += 4) {
+                        for (int q = 0; q < STAGE_SAMPLES; q += 4) {
                             const Philox4 v = philox7(hid, tid, epoch, q >> 2, g);
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
                                 const uint64_t x = static_cast<uint64_t>(v.v[i]) * nsize;
                                 low = min(low, static_cast<uint32_t>(x));
-                                k[q + i] = q + i < draws ? nbase + static_cast<int32_t>(x >> 32) : h;
+                                k[q + i] = nbase + static_cast<int32_t>(x >> 32);
                             }
                         }
                         again = low < nsize;
-#pragma unroll
-                        for (int i = 7; i >= 0; --i) to[1 + i] = k[i];
-                        to[0] = t | LIST_ATTRACT;
+                        // (the next 32 edges overwrite the padding where they continue the row)
+                        stage_edge(out, on, t | LIST_ATTRACT, k, draws, ends ? (0u - end) & (LIST_ALIGN - 1) : 0u, h);
                     } else {   // many samples per edge: straight to the list
                         if (lane < LIST_ALIGN) g.list[ebase + origin + lane] = w.stage[lane];
                         __syncwarp();
                         out = g.list + (ebase + off);
                         if (on) {
                             out[0] = t | LIST_ATTRACT;
-                            again = draw_from(hid, tid, epoch, 0, min(draws, 8u), nbase, nsize, g, out + 1);
+                            again = draw_from(hid, tid, epoch, 0, min(draws, uint32_t(STAGE_SAMPLES)), nbase, nsize, g, out + 1);
                         }
                         if (ends)
                             for (uint32_t i = end; i < round_up(end); ++i) out[i - off] = h;
