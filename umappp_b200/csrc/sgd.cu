@@ -1154,7 +1154,13 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     if (!lists_stream_) lists_stream_ = stream_get();
     cudaStream_t es = epochs_stream_, ls = overlap ? lists_stream_ : epochs_stream_;
     cudaEvent_t start = event_get(), finish = event_get(), ready = event_get(), done[2] = {event_get(), event_get()};
+    // Also on the way out of a failed call, when the streams have been waited for:
+    // the lists (2 GB at a million points) go back to the workspace cache, where
+    // the next call's come from, rather than staying with a layout that is done.
     auto settle = [&] {
+        lists_.release();
+        tasks_[0].release();
+        tasks_[1].release();
         event_put(start);
         event_put(finish);
         event_put(ready);

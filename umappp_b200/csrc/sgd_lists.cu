@@ -450,6 +450,17 @@ void InteractionLists<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s) {
 }
 
 template <typename T>
+void InteractionLists<T>::release() {
+    for (int b = 0; b < 2; ++b) {
+        list_[b].release();
+        span_[b].release();
+    }
+    cap_.release();
+    base_.release();
+    temp_.release();
+}
+
+template <typename T>
 int InteractionLists<T>::window_epochs(size_t bytes) const {
     // in an epoch about 0.28 of the edges fire, with 6 entries each (15 neighbours, 5 samples);
     // and each row has a span and a task

@@ -60,6 +60,8 @@ public:
     // Epochs per window that keep a buffer near 'bytes'.
     int window_epochs(size_t bytes) const;
     const int32_t* list(int buffer) const { return list_[buffer].get(); }
+    // Gives the buffers back to the workspace cache; the next prepare() takes new ones.
+    void release();
     const ListSpan* spans(int buffer) const { return span_[buffer].get(); }   // [epoch of the window][row]
     InteractionLists() = default;
     InteractionLists(const InteractionLists&) = delete;
