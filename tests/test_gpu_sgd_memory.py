@@ -1,4 +1,8 @@
 """Device memory of the layout epochs' interaction lists: what a layout holds between and after its runs."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -48,3 +52,29 @@ def test_layouts_keep_no_lists(umap):
     assert in_use(umap) - start <= held + MB
     del status
     assert in_use(umap) == start
+
+
+WINDOW_SCRIPT = """
+import sys
+sys.path[:0] = [%r, %r]
+import torch
+import umappp_b200
+from test_gpu_sgd_memory import layout
+status, Y = layout(umappp_b200, epochs=60, negative_sample_rate=100.0, learning_rate=0.01)
+status.run(Y, 1)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+status.run(Y)
+torch.cuda.synchronize()
+print(free - torch.cuda.mem_get_info()[0])
+"""
+
+
+def test_window_bytes_bound_the_lists(umap):
+    """100 samples per firing edge: an epoch's lists take some 55 MB, 8 epochs (which a window of 32 MB had with 5
+    samples) 430 MB per buffer.  The workspace cache keeps what a run took, so the device's free memory tells."""
+    tests = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", WINDOW_SCRIPT % (os.path.dirname(tests), tests)], capture_output=True,
+                       text=True, env=dict(os.environ, UMAPB_SGD_WINDOW_BYTES=str(256 * MB)))
+    assert r.returncode == 0, r.stderr
+    assert int(r.stdout) <= 1.25 * 256 * MB

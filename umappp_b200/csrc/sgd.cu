@@ -969,7 +969,8 @@ bool check_schedule() {
 
 // Bytes of interaction lists held at once: at a million points ten epochs (the
 // schedule state is read and written once a window: 126 ms a run with 2 GB, 135
-// with 1 GB, 124 with 4 GB).  UMAPB_SGD_WINDOW_BYTES overrides it.
+// with 1 GB, 124 with 4 GB).  Windows of several epochs stay within a quarter
+// above it, whatever the sample rate.  UMAPB_SGD_WINDOW_BYTES overrides it.
 size_t window_bytes() {
     const char* e = std::getenv("UMAPB_SGD_WINDOW_BYTES");
     return e && *e ? static_cast<size_t>(std::max(1ll, std::atoll(e))) : size_t(1) << 31;
@@ -1180,14 +1181,14 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         UMAPB_CUDA(cudaEventRecord(ready, s));
         UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
         UMAPB_CUDA(cudaStreamWaitEvent(ls, ready, 0));
-        const int window = lists_.window_epochs(overlap ? window_bytes() / 2 : window_bytes());
-        lists_.prepare(first, std::min(window, E), enext_.get(), enneg_.get(), overlap, ls);
+        const size_t bytes = overlap ? window_bytes() / 2 : window_bytes();   // of each buffer
+        lists_.prepare(first, std::min(lists_.window_epochs(0, bytes), E), enext_.get(), enneg_.get(), overlap, ls);
         int buffer = 0;
         for (int e0 = first, windows = 0; e0 < last; ++windows) {
             if (overlap) buffer = windows & 1;   // in turns one is enough
             // the buffer's last epochs are done with it
             if (overlap && windows >= 2) UMAPB_CUDA(cudaStreamWaitEvent(ls, done[buffer], 0));
-            const int W = lists_.build(buffer, enext_.get(), enneg_.get(), stream,
+            const int W = lists_.build(buffer, bytes, enext_.get(), enneg_.get(), stream,
                                        check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
             if (n > 0) {
                 tasks_[buffer].reserve(static_cast<size_t>(W) * n, ls);
@@ -1197,7 +1198,9 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
             }
             UMAPB_CUDA(cudaEventRecord(ready, ls));
             UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
-            if (e0 + W < last) lists_.prepare(e0 + W, std::min(window, last - e0 - W), enext_.get(), enneg_.get(), overlap, ls);
+            if (e0 + W < last)
+                lists_.prepare(e0 + W, std::min(lists_.window_epochs(overlap ? buffer ^ 1 : buffer, bytes), last - e0 - W),
+                               enext_.get(), enneg_.get(), overlap, ls);
             for (int e = e0; e < e0 + W && n > 0; ++e) {
                 const T epoch_t = static_cast<T>(e);
                 // alpha = lr * (1 - epoch / num_epochs) in the reference's types (optimize_layout.hpp:132-133)
@@ -1334,11 +1337,12 @@ void transform_layout(const DeviceEpochs<T>& ep, int num_dim, const T* Yref, int
     T* Yp = const_cast<T*>(vectors(Ynew, nq, new_copy));
     InteractionLists<T> lists;
     lists.setup(&ep, s);
-    const int last = ep.total_epochs, window = lists.window_epochs(window_bytes());
-    lists.prepare(0, std::min(window, last), en.get(), enn.get(), false, s);
+    const int last = ep.total_epochs;
+    const size_t bytes = window_bytes();
+    lists.prepare(0, std::min(lists.window_epochs(0, bytes), last), en.get(), enn.get(), false, s);
     for (int e0 = 0; e0 < last;) {
-        const int W = lists.build(0, en.get(), enn.get(), stream, nullptr, false, s);
-        if (e0 + W < last) lists.prepare(e0 + W, std::min(window, last - e0 - W), en.get(), enn.get(), false, s);
+        const int W = lists.build(0, bytes, en.get(), enn.get(), stream, nullptr, false, s);
+        if (e0 + W < last) lists.prepare(e0 + W, std::min(lists.window_epochs(0, bytes), last - e0 - W), en.get(), enn.get(), false, s);
         for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
             constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
             const int64_t threads = static_cast<int64_t>(nq) * G;

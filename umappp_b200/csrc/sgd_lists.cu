@@ -460,13 +460,28 @@ void InteractionLists<T>::release() {
     temp_.release();
 }
 
+// Entries of a list allocated for 'total': windows of one run differ a little,
+// and in its first epoch hardly an edge fires.
+static uint64_t list_room(uint64_t total) { return total + total / 8; }
+
 template <typename T>
-int InteractionLists<T>::window_epochs(size_t bytes) const {
-    // in an epoch about 0.28 of the edges fire, with 6 entries each (15 neighbours, 5 samples);
-    // and each row has a span and a task
-    const double per_epoch = 4.0 * 1.85 * static_cast<double>(std::max<int64_t>(ep_->nnz, 1)) +
-                             static_cast<double>(sizeof(ListSpan) + sizeof(RowTask)) * ep_->n;
-    return static_cast<int>(std::min<double>(MAX_WINDOW, std::max(1.0, static_cast<double>(bytes) / per_epoch)));
+int InteractionLists<T>::window_epochs(int buffer, size_t bytes) const {
+    double entries = per_epoch_;
+    if (entries == 0) {
+        // no window yet: about 0.28 of the edges fire in an epoch (15 neighbours), with a
+        // target and negative_sample_rate samples each, and rows are padded
+        entries = (0.28 * (1.0 + std::max(0.0, static_cast<double>(ep_->negative_sample_rate))) + 0.17) *
+                  static_cast<double>(std::max<int64_t>(ep_->nnz, 1));
+    }
+    double epochs = static_cast<double>(bytes) / epoch_bytes(entries);
+    if (full_grown(buffer, bytes)) epochs = std::min(epochs, list_[buffer].size() / entries);
+    return static_cast<int>(std::min<double>(MAX_WINDOW, std::max(1.0, epochs)));
+}
+
+// Bytes of an epoch of so many entries: they, and each row's span and task.
+template <typename T>
+double InteractionLists<T>::epoch_bytes(double entries) const {
+    return 4.0 * entries + static_cast<double>(sizeof(ListSpan) + sizeof(RowTask)) * ep_->n;
 }
 
 template <typename T>
@@ -497,8 +512,8 @@ void InteractionLists<T>::prepare(int first, int epochs, const T* enext, const T
 }
 
 template <typename T>
-int InteractionLists<T>::build(int buffer, T* enext, T* enneg, const ListStream& stream, unsigned long long* totals,
-                               bool beside_epochs, cudaStream_t s) {
+int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, const ListStream& stream,
+                               unsigned long long* totals, bool beside_epochs, cudaStream_t s) {
     if (nseg_ == 0) return epochs_;
     DevArray<int32_t>& list = list_[buffer];
     DevArray<ListSpan>& span = span_[buffer];
@@ -506,9 +521,16 @@ int InteractionLists<T>::build(int buffer, T* enext, T* enneg, const ListStream&
         UMAPB_CUDA(cudaEventSynchronize(sized_));
         const uint64_t total = *total_;
         bool fits = total / LIST_ALIGN <= UINT32_MAX;
+        per_epoch_ = static_cast<double>(std::max<uint64_t>(total, 1)) / epochs_;
+        // (more samples or firing edges than the window's length was chosen for)
+        if (epochs_ > 1 && (epoch_bytes(per_epoch_) * epochs_ > 1.125 * static_cast<double>(bytes) ||
+                            (total > list.size() && full_grown(buffer, bytes)))) {
+            prepare(first_, std::min(epochs_ - 1, window_epochs(buffer, bytes)), enext, enneg, beside_epochs, s);
+            continue;
+        }
         if (fits) {
             try {
-                if (total > list.size()) list.allocate(total + total / 16, s);   // windows of one run differ a little
+                if (total > list.size()) list.allocate(list_room(total), s);
                 span.reserve(static_cast<size_t>(epochs_) * ep_->n, s);
             } catch (const Error& e) {
                 list.release();

@@ -52,13 +52,14 @@ public:
     // run on another stream meanwhile, so the launch leaves them room.
     void prepare(int first, int epochs, const T* enext, const T* enneg, bool beside_epochs, cudaStream_t s);
     // Waits for prepare(), then enqueues the window's lists (into 'buffer') and
-    // the state at its end.  A window that does not fit the device is halved
-    // and sized again.  totals (optional, 2 per epoch from the window's first):
+    // the state at its end.  A window of several epochs is shortened and sized
+    // again where it would take more than a quarter above 'bytes', or does not
+    // fit the device.  totals (optional, 2 per epoch from the window's first):
     // [firing edges, negative samples].  Returns the epochs built.
-    int build(int buffer, T* enext, T* enneg, const ListStream& stream, unsigned long long* totals, bool beside_epochs,
-              cudaStream_t s);
-    // Epochs per window that keep a buffer near 'bytes'.
-    int window_epochs(size_t bytes) const;
+    int build(int buffer, size_t bytes, T* enext, T* enneg, const ListStream& stream, unsigned long long* totals,
+              bool beside_epochs, cudaStream_t s);
+    // Epochs of a window that takes 'buffer' up to 'bytes', by the last window built.
+    int window_epochs(int buffer, size_t bytes) const;
     const int32_t* list(int buffer) const { return list_[buffer].get(); }
     // Gives the buffers back to the workspace cache; the next prepare() takes new ones.
     void release();
@@ -72,6 +73,10 @@ private:
     const DeviceEpochs<T>* ep_ = nullptr;
     int64_t nseg_ = 0;
     int first_ = 0, epochs_ = 0;
+    double per_epoch_ = 0;         // entries of an epoch of the last window
+    double epoch_bytes(double entries) const;
+    // A buffer that holds half of the bytes it may take is not grown for the next window: that is shortened.
+    bool full_grown(int buffer, size_t bytes) const { return 8.0 * list_[buffer].size() >= static_cast<double>(bytes); }
     DevArray<int32_t> seg_row_;    // first row of each segment, nseg + 1
     DevArray<uint64_t> cap_, base_;
     DevArray<unsigned char> temp_;
