@@ -78,3 +78,32 @@ def test_window_bytes_bound_the_lists(umap):
                        text=True, env=dict(os.environ, UMAPB_SGD_WINDOW_BYTES=str(256 * MB)))
     assert r.returncode == 0, r.stderr
     assert int(r.stdout) <= 1.25 * 256 * MB
+
+
+@pytest.mark.parametrize("num_dim", [2, 3])
+def test_runs_short_of_memory(umap, monkeypatch, num_dim):
+    """With less and less device memory a run takes shorter windows, one after the other where two do not fit; where
+    even one epoch (some 6 MB here) does not, it fails and leaves the layout and the epoch as they were, so that it can
+    be run again."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("UMAPB_SGD_WINDOW_BYTES", str(64 * MB))
+    n = 20000
+    X = torch.from_numpy(oracle.gaussian_mixture(n, 10, 8, 4.0, seed=3, dtype=np.float32)).cuda()
+    Y = torch.from_numpy(np.random.default_rng(1).normal(scale=5.0, size=(n, num_dim)).astype(np.float32)).cuda()
+    start = Y.clone()
+    torch.cuda.synchronize()
+    status = umap.initialize_from_data(X, num_dim, Y, umap.Options(
+        num_epochs=30, initialize_method=umap.InitializeMethod.NONE))
+    held, failed = in_use(umap), 0
+    for room in list(np.arange(0.5, 12, 0.5)) + [12]:
+        before = umap.lib().umapb_set_workspace_limit(held + int(room * MB))
+        try:
+            status.run(Y)
+        except umap.UmapbError:
+            failed += 1
+            assert status.epoch() == 0 and torch.equal(Y, start), room
+        finally:
+            umap.lib().umapb_set_workspace_limit(before)
+        if status.epoch():
+            break
+    assert failed > 0 and status.epoch() == 30 and not torch.equal(Y, start)

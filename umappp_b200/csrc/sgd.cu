@@ -1098,7 +1098,7 @@ void SgdEngine<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s, int base_epo
         UMAPB_CUDA(cub::DeviceRadixSort::SortPairs(temp.get(), tb, key.get(), key_sorted.get(), row.get(), order_.get(),
                                                    n, 0, end_bit, s));
     }
-    lists_.setup(ep, s);
+    lists_.setup(ep, true, s);
 }
 
 template <typename T>
@@ -1140,6 +1140,7 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     const size_t values = static_cast<size_t>(n) * stride;
     const bool copied = stride != num_dim || reinterpret_cast<uintptr_t>(Y) % 16 != 0;
     DevArray<T> copy(copied ? values : 0, s);
+    DevArray<T> before;   // the layout as it was: a call that fails leaves it so, and its epochs undone
     T* Yp = copied ? copy.get() : Y;
     const int E = last - first;
     DevArray<int> counters(E, s);
@@ -1160,8 +1161,6 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     // the next call's come from, rather than staying with a layout that is done.
     auto settle = [&] {
         lists_.release();
-        tasks_[0].release();
-        tasks_[1].release();
         event_put(start);
         event_put(finish);
         event_put(ready);
@@ -1188,26 +1187,43 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
             if (overlap) buffer = windows & 1;   // in turns one is enough
             // the buffer's last epochs are done with it
             if (overlap && windows >= 2) UMAPB_CUDA(cudaStreamWaitEvent(ls, done[buffer], 0));
-            const int W = lists_.build(buffer, bytes, enext_.get(), enneg_.get(), stream,
-                                       check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
+            auto build = [&] {
+                return lists_.build(buffer, bytes, enext_.get(), enneg_.get(), stream,
+                                    check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
+            };
+            auto epochs_ahead = [&](int from, int into) { return std::min(lists_.window_epochs(into, bytes), last - from); };
+            int W = 0;
+            try {
+                W = build();
+            } catch (const Error& e) {
+                if (e.code != UMAPB_ERR_OOM || !overlap || windows == 0) throw;
+                // no memory for a second window beside the one whose epochs run: after it then
+                UMAPB_CUDA(cudaStreamSynchronize(es));
+                lists_.release(buffer ^ 1);
+                lists_.prepare(e0, epochs_ahead(e0, buffer), enext_.get(), enneg_.get(), overlap, ls);
+                W = build();
+            }
             if (n > 0) {
-                tasks_[buffer].reserve(static_cast<size_t>(W) * n, ls);
                 epoch_order_kernel<<<dim3((n - 1) / ORDER_GROUP + 1, W), EPOCH_ORDER_THREADS, 0, ls>>>(
-                    order_.get(), n, epoch_order, lists_.spans(buffer), tasks_[buffer].get());
+                    order_.get(), n, epoch_order, lists_.spans(buffer), lists_.tasks(buffer));
                 UMAPB_LAUNCH_CHECK();
             }
             UMAPB_CUDA(cudaEventRecord(ready, ls));
             UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
-            if (e0 + W < last)
-                lists_.prepare(e0 + W, std::min(lists_.window_epochs(overlap ? buffer ^ 1 : buffer, bytes), last - e0 - W),
-                               enext_.get(), enneg_.get(), overlap, ls);
+            if (e0 + W < last) {
+                if (!copied && windows == 0) {   // a later window may fail
+                    before.allocate(values, es);
+                    UMAPB_CUDA(cudaMemcpyAsync(before.get(), Y, values * sizeof(T), cudaMemcpyDeviceToDevice, es));
+                }
+                lists_.prepare(e0 + W, epochs_ahead(e0 + W, overlap ? buffer ^ 1 : buffer), enext_.get(), enneg_.get(), overlap, ls);
+            }
             for (int e = e0; e < e0 + W && n > 0; ++e) {
                 const T epoch_t = static_cast<T>(e);
                 // alpha = lr * (1 - epoch / num_epochs) in the reference's types (optimize_layout.hpp:132-133)
                 p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(epoch_t / static_cast<T>(total))));
                 for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
                     constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
-                    const RowTask* tasks = tasks_[buffer].get() + static_cast<size_t>(e - e0) * n;
+                    const RowTask* tasks = lists_.tasks(buffer) + static_cast<size_t>(e - e0) * n;
                     if (relay_rows(rows)) {
                         static const int64_t resident = resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS);
                         const int share = relay_share<G>(rows);
@@ -1240,6 +1256,7 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         cudaGetLastError();
         cudaStreamSynchronize(ls);   // nothing may still use what is released on the way out
         cudaStreamSynchronize(es);
+        if (before.size()) cudaMemcpyAsync(Y, before.get(), before.bytes(), cudaMemcpyDeviceToDevice, s);
         cudaStreamSynchronize(s);
         settle();
         throw;
@@ -1336,7 +1353,7 @@ void transform_layout(const DeviceEpochs<T>& ep, int num_dim, const T* Yref, int
     Yref = vectors(Yref, nref, ref_copy);
     T* Yp = const_cast<T*>(vectors(Ynew, nq, new_copy));
     InteractionLists<T> lists;
-    lists.setup(&ep, s);
+    lists.setup(&ep, false, s);
     const int last = ep.total_epochs;
     const size_t bytes = window_bytes();
     lists.prepare(0, std::min(lists.window_epochs(0, bytes), last), en.get(), enn.get(), false, s);

@@ -439,8 +439,9 @@ InteractionLists<T>::~InteractionLists() {
 }
 
 template <typename T>
-void InteractionLists<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s) {
+void InteractionLists<T>::setup(const DeviceEpochs<T>* ep, bool with_tasks, cudaStream_t s) {
     ep_ = ep;
+    with_tasks_ = with_tasks;
     nseg_ = ep->n > 0 ? ep->nnz / seg_target<T>() + 1 : 0;
     if (nseg_ == 0) return;
     seg_row_.allocate(nseg_ + 1, s);
@@ -450,11 +451,16 @@ void InteractionLists<T>::setup(const DeviceEpochs<T>* ep, cudaStream_t s) {
 }
 
 template <typename T>
+void InteractionLists<T>::release(int buffer) {
+    list_[buffer].release();
+    span_[buffer].release();
+    tasks_[buffer].release();
+}
+
+template <typename T>
 void InteractionLists<T>::release() {
-    for (int b = 0; b < 2; ++b) {
-        list_[b].release();
-        span_[b].release();
-    }
+    release(0);
+    release(1);
     cap_.release();
     base_.release();
     temp_.release();
@@ -490,10 +496,27 @@ void InteractionLists<T>::prepare(int first, int epochs, const T* enext, const T
     first_ = first;
     epochs_ = std::min(epochs, MAX_WINDOW);
     if (nseg_ == 0) return;
-    const int64_t cells = nseg_ * epochs_;
-    require(cells < INT32_MAX, "too many edges for the schedule's segments", UMAPB_ERR_OVERFLOW);
-    cap_.reserve(cells + 1, s);
-    base_.reserve(cells + 1, s);
+    int64_t cells = 0;
+    size_t tb = 0;
+    for (;; epochs_ = (epochs_ + 1) / 2) {
+        cells = nseg_ * epochs_;
+        if (cells >= INT32_MAX) {
+            require(epochs_ > 1, "too many edges for the schedule's segments", UMAPB_ERR_OVERFLOW);
+            continue;
+        }
+        try {
+            cap_.reserve(cells + 1, s);
+            base_.reserve(cells + 1, s);
+            UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cap_.get(), base_.get(), static_cast<int>(cells + 1), s));
+            temp_.reserve(tb, s);
+            break;
+        } catch (const Error& e) {
+            cap_.release();
+            base_.release();
+            temp_.release();
+            if (e.code != UMAPB_ERR_OOM || epochs_ == 1) throw;
+        }
+    }
     UMAPB_CUDA(cudaMemsetAsync(cap_.get() + cells, 0, sizeof(uint64_t), s));
     GenArgs<T> g = gen_args(*ep_, seg_row_.get(), nseg_, first_, epochs_);
     g.enext = const_cast<T*>(enext);   // read only while sizing
@@ -501,9 +524,6 @@ void InteractionLists<T>::prepare(int first, int epochs, const T* enext, const T
     g.cap = cap_.get();
     schedule_kernel<T, false><<<gen_grid(nseg_, beside_epochs), GEN_WARPS * 32, 0, s>>>(g);
     UMAPB_LAUNCH_CHECK();
-    size_t tb = 0;
-    UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cap_.get(), base_.get(), static_cast<int>(cells + 1), s));
-    temp_.reserve(tb, s);
     UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(temp_.get(), tb, cap_.get(), base_.get(), static_cast<int>(cells + 1), s));
     if (!total_) total_ = static_cast<uint64_t*>(pinned_get());
     if (!sized_) sized_ = event_get();
@@ -516,7 +536,6 @@ int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, con
                                unsigned long long* totals, bool beside_epochs, cudaStream_t s) {
     if (nseg_ == 0) return epochs_;
     DevArray<int32_t>& list = list_[buffer];
-    DevArray<ListSpan>& span = span_[buffer];
     while (true) {
         UMAPB_CUDA(cudaEventSynchronize(sized_));
         const uint64_t total = *total_;
@@ -531,10 +550,10 @@ int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, con
         if (fits) {
             try {
                 if (total > list.size()) list.allocate(list_room(total), s);
-                span.reserve(static_cast<size_t>(epochs_) * ep_->n, s);
+                span_[buffer].reserve(static_cast<size_t>(epochs_) * ep_->n, s);
+                if (with_tasks_) tasks_[buffer].reserve(static_cast<size_t>(epochs_) * ep_->n, s);
             } catch (const Error& e) {
-                list.release();
-                span.release();
+                release(buffer);
                 if (e.code != UMAPB_ERR_OOM || epochs_ == 1) throw;
                 fits = false;
             }
@@ -548,7 +567,7 @@ int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, con
     g.enneg = enneg;
     g.base = base_.get();
     g.list = list.get();
-    g.span = span.get();
+    g.span = span_[buffer].get();
     g.stream = stream;
     g.totals = totals;
     for (uint32_t r = 0; r < 7; ++r) {

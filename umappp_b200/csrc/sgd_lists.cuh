@@ -46,10 +46,12 @@ struct ListStream {
 template <typename T>
 class InteractionLists {
 public:
-    void setup(const DeviceEpochs<T>* ep, cudaStream_t s);
+    // with_tasks: the buffers also have room for the epochs' row tasks.
+    void setup(const DeviceEpochs<T>* ep, bool with_tasks, cudaStream_t s);
     // Enqueues the sizing of the window [first, first + epochs) from the state
     // (enext, enneg) at 'first', which stays as it is.  beside_epochs: epochs
-    // run on another stream meanwhile, so the launch leaves them room.
+    // run on another stream meanwhile, so the launch leaves them room.  Fewer
+    // epochs are sized where the device has no memory for more.
     void prepare(int first, int epochs, const T* enext, const T* enneg, bool beside_epochs, cudaStream_t s);
     // Waits for prepare(), then enqueues the window's lists (into 'buffer') and
     // the state at its end.  A window of several epochs is shortened and sized
@@ -61,8 +63,10 @@ public:
     // Epochs of a window that takes 'buffer' up to 'bytes', by the last window built.
     int window_epochs(int buffer, size_t bytes) const;
     const int32_t* list(int buffer) const { return list_[buffer].get(); }
-    // Gives the buffers back to the workspace cache; the next prepare() takes new ones.
+    // Gives a buffer, or all memory, back to the workspace cache; prepare() and build() take it anew.
+    void release(int buffer);
     void release();
+    RowTask* tasks(int buffer) const { return tasks_[buffer].get(); }   // [epoch of the window][position]
     const ListSpan* spans(int buffer) const { return span_[buffer].get(); }   // [epoch of the window][row]
     InteractionLists() = default;
     InteractionLists(const InteractionLists&) = delete;
@@ -82,6 +86,8 @@ private:
     DevArray<unsigned char> temp_;
     DevArray<int32_t> list_[2];
     DevArray<ListSpan> span_[2];
+    DevArray<RowTask> tasks_[2];
+    bool with_tasks_ = false;
     uint64_t* total_ = nullptr;    // pinned host word
     cudaEvent_t sized_ = nullptr;
 };

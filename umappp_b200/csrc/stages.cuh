@@ -223,7 +223,6 @@ private:
     static bool default_epoch_order();
     const DeviceEpochs<T>* ep_ = nullptr;
     InteractionLists<T> lists_;
-    DevArray<RowTask> tasks_[2];      // per list buffer, [epoch of the window][position]: the rows in claim order
     cudaStream_t epochs_stream_ = nullptr, lists_stream_ = nullptr;
     const int32_t* inst_start_ = nullptr;
     int32_t num_inst_ = 1;
