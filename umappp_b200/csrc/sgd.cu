@@ -969,12 +969,15 @@ bool check_schedule() {
 
 // Bytes of interaction lists held at once: at a million points ten epochs (the
 // schedule state is read and written once a window: 126 ms a run with 2 GB, 135
-// with 1 GB, 124 with 4 GB).  Windows of several epochs stay within a quarter
+// with 1 GB, 124 with 4 GB).  Windows of several epochs stay within an eighth
 // above it, whatever the sample rate.  UMAPB_SGD_WINDOW_BYTES overrides it.
 size_t window_bytes() {
     const char* e = std::getenv("UMAPB_SGD_WINDOW_BYTES");
     return e && *e ? static_cast<size_t>(std::max(1ll, std::atoll(e))) : size_t(1) << 31;
 }
+
+// Calls of at most this many epochs have their lists read ahead (SgdEngine::run).
+constexpr int FEW_EPOCHS = 8;
 
 int sm_count() {
     static int count = 0;
@@ -1159,8 +1162,10 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     // Also on the way out of a failed call, when the streams have been waited for:
     // the lists (2 GB at a million points) go back to the workspace cache, where
     // the next call's come from, rather than staying with a layout that is done.
+    // (Read ahead for a program that runs a few epochs at a time, a window stays.)
     auto settle = [&] {
-        lists_.release();
+        if (ahead_.epochs > 0) lists_.release(ahead_.buffer ^ 1);
+        else lists_.release();
         event_put(start);
         event_put(finish);
         event_put(ready);
@@ -1169,8 +1174,24 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     };
     try {
         UMAPB_CUDA(cudaEventRecord(start, s));
-        if (state_epoch_ != first) state_at(first, enext_.get(), enneg_.get(), s);
+        // A window that the call before has begun, and where the schedule state stands
+        ListWindow w = ahead_;
+        const bool begun = w.epochs > 0 && w.seed == seed && w.first <= first && first < w.first + w.epochs &&
+                           state_epoch_ == w.first + w.epochs && !check;
+        int from = begun ? w.first + w.epochs : first;
+        ahead_ = ListWindow();
+        if (!begun) {
+            if (w.epochs > 0) lists_.release(w.buffer);
+            if (state_epoch_ != first) state_at(first, enext_.get(), enneg_.get(), s);
+        }
         state_epoch_ = -1;   // until the call has succeeded
+        // Calls of a few epochs, one after the other (a program that shows the layout
+        // as it goes): every window is as long as two before it, and what is left of
+        // it is kept.  (20 calls of one epoch, ms: a million points 16.6 without,
+        // 300 points 2.0.)
+        const bool few = !check && E <= FEW_EPOCHS;
+        const int least = few && first == run_end_ ? std::min(2 * std::max(least_, E), MAX_WINDOW) : 0;
+        run_end_ = -1;
         counters.zero(s);
         if (check) totals.zero(s);
         if (copied && n > 0) {
@@ -1181,49 +1202,61 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
         UMAPB_CUDA(cudaStreamWaitEvent(ls, ready, 0));
         const size_t bytes = overlap ? window_bytes() / 2 : window_bytes();   // of each buffer
-        lists_.prepare(first, std::min(lists_.window_epochs(0, bytes), E), enext_.get(), enneg_.get(), overlap, ls);
-        int buffer = 0;
-        for (int e0 = first, windows = 0; e0 < last; ++windows) {
-            if (overlap) buffer = windows & 1;   // in turns one is enough
-            // the buffer's last epochs are done with it
-            if (overlap && windows >= 2) UMAPB_CUDA(cudaStreamWaitEvent(ls, done[buffer], 0));
-            auto build = [&] {
-                return lists_.build(buffer, bytes, enext_.get(), enneg_.get(), stream,
-                                    check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
-            };
-            auto epochs_ahead = [&](int from, int into) { return std::min(lists_.window_epochs(into, bytes), last - from); };
-            int W = 0;
-            try {
-                W = build();
-            } catch (const Error& e) {
-                if (e.code != UMAPB_ERR_OOM || !overlap || windows == 0) throw;
-                // no memory for a second window beside the one whose epochs run: after it then
-                UMAPB_CUDA(cudaStreamSynchronize(es));
-                lists_.release(buffer ^ 1);
-                lists_.prepare(e0, epochs_ahead(e0, buffer), enext_.get(), enneg_.get(), overlap, ls);
-                W = build();
+        // epochs of the window from 'at' on: the call's, or beyond them as far as is read ahead
+        auto window = [&](int at, int into) {
+            const int fit = lists_.window_epochs(into, bytes);
+            const int more = std::min(least, std::min(lists_.window_epochs(into, bytes / 2), total - at));   // (half a buffer at most)
+            return std::min(fit, std::max(last - at, more));
+        };
+        bool used[2] = {false, false};   // by epochs of this call
+        int buffer = begun ? w.buffer : 0;
+        auto after = [&] { return overlap && used[buffer] ? buffer ^ 1 : buffer; };   // in turns one is enough
+        if (from < last && !begun) lists_.prepare(from, window(from, buffer), enext_.get(), enneg_.get(), overlap, ls);
+        for (int e0 = first; e0 < last;) {
+            if (e0 == from) {
+                buffer = after();
+                // the buffer's last epochs are done with it
+                if (overlap && used[buffer]) UMAPB_CUDA(cudaStreamWaitEvent(ls, done[buffer], 0));
+                auto build = [&] {
+                    return lists_.build(buffer, bytes, enext_.get(), enneg_.get(), stream,
+                                        check ? totals.get() + 2 * (e0 - first) : nullptr, overlap, ls);
+                };
+                w = ListWindow{e0, 0, buffer, seed};
+                try {
+                    w.epochs = build();
+                } catch (const Error& e) {
+                    if (e.code != UMAPB_ERR_OOM || !used[buffer ^ 1]) throw;
+                    // no memory for a second window beside the one whose epochs run: after it then
+                    UMAPB_CUDA(cudaStreamSynchronize(es));
+                    lists_.release(buffer ^ 1);
+                    lists_.prepare(e0, window(e0, buffer), enext_.get(), enneg_.get(), overlap, ls);
+                    w.epochs = build();
+                }
+                from = e0 + w.epochs;
+                if (n > 0) {
+                    epoch_order_kernel<<<dim3((n - 1) / ORDER_GROUP + 1, w.epochs), EPOCH_ORDER_THREADS, 0, ls>>>(
+                        order_.get(), n, epoch_order, lists_.spans(buffer), lists_.tasks(buffer));
+                    UMAPB_LAUNCH_CHECK();
+                }
+                UMAPB_CUDA(cudaEventRecord(ready, ls));
+                UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
             }
-            if (n > 0) {
-                epoch_order_kernel<<<dim3((n - 1) / ORDER_GROUP + 1, W), EPOCH_ORDER_THREADS, 0, ls>>>(
-                    order_.get(), n, epoch_order, lists_.spans(buffer), lists_.tasks(buffer));
-                UMAPB_LAUNCH_CHECK();
-            }
-            UMAPB_CUDA(cudaEventRecord(ready, ls));
-            UMAPB_CUDA(cudaStreamWaitEvent(es, ready, 0));
-            if (e0 + W < last) {
-                if (!copied && windows == 0) {   // a later window may fail
+            used[buffer] = true;
+            if (from < last) {
+                if (!copied && before.size() == 0) {   // a later window may fail
                     before.allocate(values, es);
                     UMAPB_CUDA(cudaMemcpyAsync(before.get(), Y, values * sizeof(T), cudaMemcpyDeviceToDevice, es));
                 }
-                lists_.prepare(e0 + W, epochs_ahead(e0 + W, overlap ? buffer ^ 1 : buffer), enext_.get(), enneg_.get(), overlap, ls);
+                lists_.prepare(from, window(from, after()), enext_.get(), enneg_.get(), overlap, ls);
             }
-            for (int e = e0; e < e0 + W && n > 0; ++e) {
+            const int e1 = std::min(from, last);
+            for (int e = e0; e < e1 && n > 0; ++e) {
                 const T epoch_t = static_cast<T>(e);
                 // alpha = lr * (1 - epoch / num_epochs) in the reference's types (optimize_layout.hpp:132-133)
                 p.alpha = static_cast<T>(static_cast<double>(lr) * (1.0 - static_cast<double>(epoch_t / static_cast<T>(total))));
                 for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
                     constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
-                    const RowTask* tasks = lists_.tasks(buffer) + static_cast<size_t>(e - e0) * n;
+                    const RowTask* tasks = lists_.tasks(buffer) + static_cast<size_t>(e - w.first) * n;
                     if (relay_rows(rows)) {
                         static const int64_t resident = resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS);
                         const int share = relay_share<G>(rows);
@@ -1240,7 +1273,7 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
                 UMAPB_LAUNCH_CHECK();
             }
             UMAPB_CUDA(cudaEventRecord(done[buffer], es));
-            e0 += W;
+            e0 = e1;
         }
         UMAPB_CUDA(cudaStreamWaitEvent(s, done[buffer], 0));   // the last window's: the lists came before it
         if (copied && n > 0) {
@@ -1252,6 +1285,10 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         float ms = 0;
         UMAPB_CUDA(cudaEventElapsedTime(&ms, start, finish));
         if (ms_sgd) *ms_sgd = ms;
+        state_epoch_ = from;
+        if (from > last) ahead_ = w;
+        run_end_ = last;
+        least_ = least;
     } catch (...) {
         cudaGetLastError();
         cudaStreamSynchronize(ls);   // nothing may still use what is released on the way out
@@ -1262,7 +1299,6 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
         throw;
     }
     settle();
-    state_epoch_ = last;
     if (check) {
         std::vector<int64_t> want(2 * static_cast<size_t>(E));
         counts(first, last, want.data(), s);

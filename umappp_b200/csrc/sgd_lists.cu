@@ -466,9 +466,11 @@ void InteractionLists<T>::release() {
     temp_.release();
 }
 
-// Entries of a list allocated for 'total': windows of one run differ a little,
-// and in its first epoch hardly an edge fires.
-static uint64_t list_room(uint64_t total) { return total + total / 8; }
+// Entries of a list allocated for a window's 'total' of at most 'most' bytes:
+// windows of one run differ a little, and in its first epoch hardly an edge fires.
+static uint64_t list_room(uint64_t total, double most) {
+    return std::max(total, std::min(total + total / 8, static_cast<uint64_t>(std::max(0.0, most) / 4)));
+}
 
 template <typename T>
 int InteractionLists<T>::window_epochs(int buffer, size_t bytes) const {
@@ -542,14 +544,15 @@ int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, con
         bool fits = total / LIST_ALIGN <= UINT32_MAX;
         per_epoch_ = static_cast<double>(std::max<uint64_t>(total, 1)) / epochs_;
         // (more samples or firing edges than the window's length was chosen for)
-        if (epochs_ > 1 && (epoch_bytes(per_epoch_) * epochs_ > 1.125 * static_cast<double>(bytes) ||
+        const double most = 1.125 * static_cast<double>(bytes);
+        if (epochs_ > 1 && (epoch_bytes(per_epoch_) * epochs_ > most ||
                             (total > list.size() && full_grown(buffer, bytes)))) {
             prepare(first_, std::min(epochs_ - 1, window_epochs(buffer, bytes)), enext, enneg, beside_epochs, s);
             continue;
         }
         if (fits) {
             try {
-                if (total > list.size()) list.allocate(list_room(total), s);
+                if (total > list.size()) list.allocate(list_room(total, most - epoch_bytes(0) * epochs_), s);
                 span_[buffer].reserve(static_cast<size_t>(epochs_) * ep_->n, s);
                 if (with_tasks_) tasks_[buffer].reserve(static_cast<size_t>(epochs_) * ep_->n, s);
             } catch (const Error& e) {

@@ -55,7 +55,7 @@ public:
     void prepare(int first, int epochs, const T* enext, const T* enneg, bool beside_epochs, cudaStream_t s);
     // Waits for prepare(), then enqueues the window's lists (into 'buffer') and
     // the state at its end.  A window of several epochs is shortened and sized
-    // again where it would take more than a quarter above 'bytes', or does not
+    // again where it would take more than an eighth above 'bytes', or does not
     // fit the device.  totals (optional, 2 per epoch from the window's first):
     // [firing edges, negative samples].  Returns the epochs built.
     int build(int buffer, size_t bytes, T* enext, T* enneg, const ListStream& stream, unsigned long long* totals,

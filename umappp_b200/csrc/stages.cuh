@@ -230,6 +230,13 @@ private:
     DevArray<T> enext_, enneg_;    // schedule state at state_epoch_
     DevArray<int32_t> order_;      // rows in the run's claim order
     int state_epoch_ = 0;          // epoch the state arrays describe
+    // Lists of the epochs [first, first + epochs), in a buffer of lists_.
+    struct ListWindow {
+        int first = 0, epochs = 0, buffer = 0;
+        uint64_t seed = 0;
+    };
+    ListWindow ahead_;             // read ahead by the last run() (epochs 0: none)
+    int run_end_ = -1, least_ = 0; // where it ended, and the epochs of its windows at least
 };
 
 // ---- adjoint (adjoint.cu) ----------------------------------------------------
