@@ -116,3 +116,26 @@ def test_unaligned_layout(umap, num_dim):
         out.append(store.cpu().numpy()[offset:offset + Y.size].copy())
         assert np.all(np.delete(store.cpu().numpy(), np.arange(offset, offset + Y.size)) == 0)
     assert np.array_equal(out[0], out[1])
+
+
+def test_fewer_edges_take_no_longer(umap):
+    """Three million points of which nearly all have no edge: a thousand edges in all, or four hundred thousand."""
+    import time
+
+    n, rng = 3000000, np.random.default_rng(4)
+    seconds = []
+    for edges in (1000, 400000):
+        count = np.zeros(n, dtype=np.int64)
+        count[np.sort(rng.choice(n, edges // 10, replace=False))] = 10
+        g = oracle.CSR(np.concatenate([[0], np.cumsum(count)]), rng.integers(0, n, edges).astype(np.int32),
+                       rng.uniform(0.1, 1.0, edges).astype(np.float32))
+        ep = oracle.similarities_to_epochs(g, 200, 5.0)
+        Y = np.zeros((n, 2), dtype=np.float32)
+        best = 1e9
+        for _ in range(3):
+            dev = device_epochs(umap, ep)
+            t = time.perf_counter()
+            umap.optimize_layout(2, Y, dev, 1.577, 0.895, 1.0, 1.0, 99, 200, 5.0)
+            best = min(best, time.perf_counter() - t)
+        seconds.append(best)
+    assert seconds[0] <= 1.2 * seconds[1], seconds

@@ -173,13 +173,7 @@ __global__ void __launch_bounds__(GEN_WARPS * 32, GEN_BLOCKS) schedule_kernel(co
         uint64_t base = 0, entries = 0, fired = 0, drawn = 0;
         uint32_t pos_of = 0;
         int32_t head_of = -1;
-        if (FILL) {
-            if (lane < g.epochs) base = g.base[lane * g.nseg + s];
-            for (int e = 0; e < g.epochs; ++e)
-                for (int64_t r = int64_t(r0) + lane; r < r1; r += 32)
-                    g.span[static_cast<int64_t>(e) * g.nrows + r] = ListSpan{0, 0};
-            __syncwarp();
-        }
+        if (FILL && lane < g.epochs) base = g.base[lane * g.nseg + s];
         for (int64_t c = j0; c < j1; c += SEG) {
             const int m = static_cast<int>(j1 - c < SEG ? j1 - c : SEG);
             for (int i = lane; i < m; i += 32) {
@@ -481,7 +475,8 @@ int InteractionLists<T>::window_epochs(int buffer, size_t bytes) const {
         entries = (0.28 * (1.0 + std::max(0.0, static_cast<double>(ep_->negative_sample_rate))) + 0.17) *
                   static_cast<double>(std::max<int64_t>(ep_->nnz, 1));
     }
-    double epochs = static_cast<double>(bytes) / epoch_bytes(entries);
+    // (a sixteenth above, once the entries are known: windows as long as the estimate's)
+    double epochs = (per_epoch_ == 0 ? 1.0 : 1.0625) * static_cast<double>(bytes) / epoch_bytes(entries);
     if (full_grown(buffer, bytes)) epochs = std::min(epochs, list_[buffer].size() / entries);
     return static_cast<int>(std::min<double>(MAX_WINDOW, std::max(1.0, epochs)));
 }
@@ -577,6 +572,9 @@ int InteractionLists<T>::build(int buffer, size_t bytes, T* enext, T* enneg, con
         g.key0[r] = stream.k0 + r * 0x9E3779B9u;
         g.key1[r] = stream.k1 + r * 0xBB67AE85u;
     }
+    // Rows that fire nothing keep an empty span.  (Not cleared by the segments' warps: the
+    // rows without edges between two others are all one segment's.)
+    UMAPB_CUDA(cudaMemsetAsync(span_[buffer].get(), 0, sizeof(ListSpan) * static_cast<size_t>(epochs_) * ep_->n, s));
     schedule_kernel<T, true><<<gen_grid(nseg_, beside_epochs), GEN_WARPS * 32, 0, s>>>(g);
     UMAPB_LAUNCH_CHECK();
     return epochs_;
