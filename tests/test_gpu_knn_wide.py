@@ -56,3 +56,47 @@ def test_query_far_from_references(umap):
     X = oracle.gaussian_mixture(4400, 12, 4, 3.0, seed=9, dtype=np.float32)
     new = X[4100:] + np.float32(3000.0)
     check(*umap.knn_query(X[:4100], new, 10), *oracle.knn_query(X[:4100], new, 10))
+
+
+def far(n, dim, seed):
+    """Points a thousand units from the origin: the tensor cores' bound certifies no query."""
+    return oracle.gaussian_mixture(n, dim, 4, 3.0, seed=seed, dtype=np.float32) + np.float32(1000.0)
+
+
+# sizes around the blocks of 128 queries and 32 points, dimensions around 32 columns
+@pytest.mark.parametrize("n,dim,k", [(33, 3, 15), (129, 32, 8), (1000, 33, 15), (2000, 10, 24), (3001, 20, 40), (1500, 40, 119), (2500, 4, 57)])
+def test_knn_far_from_origin(umap, n, dim, k):
+    X = far(n, dim, n + k)
+    check(*umap.knn(X, k), *oracle.knn(X, k))
+
+
+@pytest.mark.parametrize("nref,nq,dim,k", [(1024, 1, 5, 15), (4100, 300, 12, 15), (4100, 129, 40, 30), (2000, 40, 8, 110)])
+def test_query_far_from_origin(umap, nref, nq, dim, k):
+    X = far(nref + nq, dim, nref + k)
+    check(*umap.knn_query(X[:nref], X[nref:], k), *oracle.knn_query(X[:nref], X[nref:], k))
+
+
+@pytest.mark.parametrize("copies,k", [(1, 20), (100, 20), (140, 20), (100, 60), (240, 60), (270, 60)])   # within and beyond the 128 (256) points collected
+def test_knn_far_copies(umap, copies, k):
+    X = np.repeat(far(1400 // copies, 6, 3), copies, axis=0)
+    idx, dist = umap.knn(X, k)
+    ridx, rdist = oracle.knn(X, k)
+    np.testing.assert_array_equal(idx, ridx)   # FP64 distances of equal points are equal: the lower index first
+    np.testing.assert_allclose(dist.astype(np.float64), rdist, rtol=1e-6, atol=1e-30)
+
+
+def test_far_from_origin_costs_little(umap):
+    """20,000 x 20 points around the origin and a thousand units away, 60 neighbours."""
+    import time
+
+    X = oracle.gaussian_mixture(20000, 20, 10, 4.0, seed=1, dtype=np.float32)
+    seconds = []
+    for Z in (X, X + np.float32(1000.0)):
+        umap.knn(Z, 60)
+        best = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            umap.knn(Z, 60)
+            best = min(best, time.perf_counter() - t)
+        seconds.append(best)
+    assert seconds[1] <= 3 * seconds[0], seconds

@@ -233,7 +233,8 @@ __device__ __forceinline__ double distance2(const float* __restrict__ x, const f
 
 // FP64 rescoring of the FP32 candidates of every query: keeps the best k by
 // (FP64 distance, index) and flags queries whose candidate set may miss a
-// true neighbour.  A query's candidates are 'lists' lists of list_len entries
+// true neighbour (others = 0: never).  A query's results go to row 'slot', or
+// q - out_row0.  A query's candidates are 'lists' lists of list_len entries
 // (32 PER in all at most), each the nearest of its part of the points in
 // ascending FP32 order.  One warp per query, a candidate (or PER) per lane:
 // bound by the candidates' rows, read from L2 a row per lane.  (A thread per
@@ -244,9 +245,10 @@ template <int PER>
 __global__ void __launch_bounds__(RESCORE_WARPS * 32)
     knn_rescore_kernel(const float* __restrict__ data, int32_t others, int32_t dim, int32_t k,
                        const int32_t* __restrict__ queries, int32_t nq, int lists, int list_len, int cand_by_slot,
-                       int out_by_slot, const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_d2,
+                       int out_by_slot, int32_t out_row0, const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_d2,
                        int32_t* __restrict__ out_idx, float* __restrict__ out_dist, double* __restrict__ out_dist64,
-                       int32_t* __restrict__ redo, int32_t* __restrict__ redo_count, const float* __restrict__ norms,
+                       int32_t* __restrict__ redo, double* __restrict__ redo_kth, int32_t* __restrict__ redo_count,
+                       const float* __restrict__ norms,
                        const unsigned int* __restrict__ norm_max_bits, double tc_rel,
                        unsigned int* __restrict__ tc_err_bits) {
     const int lane = threadIdx.x & 31;
@@ -297,12 +299,13 @@ __global__ void __launch_bounds__(RESCORE_WARPS * 32)
     if (lane == 0 && !full_list && !certain) {
         const int32_t r = atomicAdd(redo_count, 1);
         redo[r] = out_by_slot ? slot : q;   // a slot when the output is by slot, else the data row
+        if (redo_kth) redo_kth[r] = kth;    // k points are at least as near as that
     }
     if (err_scale > 0.0) {
         for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
         if (lane == 0 && worst > 0.0f) atomicMax(tc_err_bits, __float_as_uint(worst));
     }
-    const size_t orow = static_cast<size_t>(out_by_slot ? slot : q) * k;
+    const size_t orow = static_cast<size_t>(out_by_slot ? slot : q - out_row0) * k;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int c = 32 * i + lane;
@@ -351,6 +354,142 @@ void run_f64(const T* data, int32_t n, int32_t dim, int32_t k, const int32_t* qu
     knn_emit_f64_kernel<T, KCAP><<<(nq + 127) / 128, 128, 0, s>>>(nq, queries, out_rows, k, ci.get(), cd.get(), out_idx,
                                                                   out_dist, out_dist64);
     UMAPB_LAUNCH_CHECK();
+}
+
+// ---- uncertain queries ----
+// A query whose candidates leave its k-th neighbour open: what they do tell is a
+// distance within which k points lie (kth).  All points that may be that near are
+// collected -- by FP32 differences, with their rounding in the bound -- and rescored
+// in FP64.  Where the tensor cores' bound certifies nothing (data far from the
+// origin, or one far outlier) that is every query: 20,000 x 20 points with an
+// offset of 1000, k = 15, 30 and 60: 4.0, 5.5 and 8.9 ms in all (the FP64 search of
+// every query, a list per thread: 7.2, 22.5 and 112.7; candidates by FP32
+// differences on CUDA cores in the first place: 18.0 and 85.6 for 30 and 60).
+// Collected are up to 128 points per query (256 for more than 56 neighbours);
+// queries with more of them, ties mostly, are searched in FP64.
+constexpr int32_t WITHIN_PLACES = 1 << 23;   // of the queries taken at a time (64 MB)
+
+// Thread = query, blockIdx.y = stretch of the points.
+template <int LIST>
+__global__ void __launch_bounds__(KNN_BLOCK)
+    knn_within_kernel(const float* __restrict__ data, int32_t n, int32_t dim, const int32_t* __restrict__ queries,
+                      int32_t nq, const double* __restrict__ kth, int32_t stretch, int32_t* __restrict__ list,
+                      int32_t* __restrict__ count) {
+    __shared__ float qs[CH][KNN_BLOCK];
+    __shared__ float ps[PT][CH + 1];
+    const int tid = threadIdx.x;
+    const int32_t slot = blockIdx.x * KNN_BLOCK + tid;
+    const bool active = slot < nq;
+    const int32_t q = active ? queries[slot] : 0;
+    float bound = -1.0f;
+    if (active) {
+        const double d2 = kth[slot];
+        const double rel = (dim + 2) * 1.2e-7 * 2.0;   // as in the certainty check
+        // (the addition: squares of differences below 1e-19 lose bits)
+        if (d2 < CUDART_INF) bound = __double2float_ru(d2 * (1.0 + rel) + 1e-36);
+        else if (blockIdx.y == 0) atomicAdd(&count[slot], LIST + 1);   // fewer than k candidates
+    }
+    const int32_t first = blockIdx.y * stretch;   // (a multiple of PT)
+    const int32_t last = static_cast<int32_t>(min(static_cast<int64_t>(n), static_cast<int64_t>(first) + stretch));
+    for (int32_t base = first; base < last; base += PT) {
+        float acc[PT];
+#pragma unroll
+        for (int p = 0; p < PT; ++p) acc[p] = 0;
+        for (int c0 = 0; c0 < dim; c0 += CH) {
+            const int cw = min(CH, dim - c0);
+            __syncthreads();
+            if (dim > CH || base == first)
+                for (int c = 0; c < cw; ++c) qs[c][tid] = data[static_cast<size_t>(q) * dim + c0 + c];
+            for (int e = tid; e < PT * CH; e += KNN_BLOCK) {
+                const int p = e / CH, c = e % CH;
+                const int32_t j = base + p;
+                ps[p][c] = (j < last && c < cw) ? data[static_cast<size_t>(j) * dim + c0 + c] : 0.0f;
+            }
+            __syncthreads();
+            for (int c = 0; c < cw; ++c) {
+                const float qv = qs[c][tid];
+#pragma unroll
+                for (int p = 0; p < PT; ++p) add_sq(acc[p], qv - ps[p][c]);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < PT; ++p) {
+            const int32_t j = base + p;
+            if (acc[p] <= bound && j < last && j != q) {
+                const int at = atomicAdd(&count[slot], 1);
+                if (at < LIST) list[static_cast<size_t>(slot) * LIST + at] = j;
+            }
+        }
+    }
+}
+
+// The queries with more points within reach than their lists hold.
+__global__ void knn_crowded_kernel(int32_t nq, int32_t places, const int32_t* __restrict__ count, const int32_t* __restrict__ queries,
+                                   int32_t row0, int32_t* __restrict__ crowded, int32_t* __restrict__ rows,
+                                   int32_t* __restrict__ num) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
+        if (count[i] > places) {
+            const int32_t at = atomicAdd(num, 1);
+            crowded[at] = queries[i];
+            rows[at] = queries[i] - row0;
+        }
+    }
+}
+
+// Exact search of 'nq' queries (data rows) among the data rows [0, n), k of
+// which are known to lie within kth; results to rows query - row0.
+template <int LIST>
+void run_within_lists(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
+                const double* kth, int32_t row0, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
+    int32_t batch = std::min(nq, WITHIN_PLACES / LIST);
+    DevArray<int32_t> list, count, crowded, rows, num(1, s);
+    DevArray<float> unused;   // the rescoring's FP32 distances
+    for (;; batch = (batch + 3) / 4) {
+        try {
+            list.allocate(static_cast<size_t>(batch) * LIST, s);
+            unused.allocate(static_cast<size_t>(batch) * LIST, s);
+            count.allocate(batch, s);
+            crowded.allocate(batch, s);
+            rows.allocate(batch, s);
+            break;
+        } catch (const Error& e) {
+            list.release();
+            if (e.code != UMAPB_ERR_OOM || batch <= KNN_BLOCK) throw;
+        }
+    }
+    for (int32_t at = 0; at < nq; at += batch) {
+        const int32_t m = std::min(batch, nq - at);
+        const int32_t* q = queries + at;
+        UMAPB_CUDA(cudaMemsetAsync(list.get(), 0xff, list.bytes(), s));
+        count.zero(s);
+        num.zero(s);
+        // stretches so that the device is filled four times over
+        const int32_t blocks = (m + KNN_BLOCK - 1) / KNN_BLOCK, tiles = (n - 1) / PT + 1;
+        const int32_t parts = std::min(tiles, std::max(1, 4 * 4 * 148 / blocks));
+        const int32_t stretch = (tiles + parts - 1) / parts * PT;
+        knn_within_kernel<LIST><<<dim3(blocks, (tiles - 1) / (stretch / PT) + 1), KNN_BLOCK, 0, s>>>(data, n, dim, q, m, kth + at,
+                                                                                         stretch, list.get(), count.get());
+        UMAPB_LAUNCH_CHECK();
+        knn_rescore_kernel<LIST / 32><<<rescore_grid(m), RESCORE_WARPS * 32, 0, s>>>(
+            data, 0, dim, k, q, m, 1, LIST, 1, 0, row0, list.get(), unused.get(), out_idx, out_dist, out_dist64,
+            nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr);
+        UMAPB_LAUNCH_CHECK();
+        knn_crowded_kernel<<<grid_for(m, 256), 256, 0, s>>>(m, LIST, count.get(), q, row0, crowded.get(), rows.get(), num.get());
+        UMAPB_LAUNCH_CHECK();
+        int32_t nc = 0;
+        UMAPB_CUDA(cudaMemcpyAsync(&nc, num.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        UMAPB_SYNC(s);
+        if (nc == 0) continue;
+        if (k <= 16) run_f64<float, 16>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
+        else if (k <= 32) run_f64<float, 32>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
+        else if (k <= 64) run_f64<float, 64>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
+        else run_f64<float, 128>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
+    }
+}
+void run_within(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
+                const double* kth, int32_t row0, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
+    if (k <= 56) run_within_lists<128>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s);
+    else run_within_lists<256>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s);
 }
 
 __global__ void norm_max_kernel(int32_t n, const float* __restrict__ norms, unsigned int* __restrict__ out) {
@@ -451,14 +590,15 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
         }
     }
     DevArray<int32_t> redo(std::max(nq, 1), s), redo_count(1, s);
+    DevArray<double> redo_kth(std::max(nq, 1), s);
     redo_count.zero(s);
     DevArray<unsigned int> tc_err(1, s);
     tc_err.zero(s);
     if (nq > 0) {
         knn_rescore_kernel<per_lane<KCAP>()><<<rescore_grid(nq), RESCORE_WARPS * 32, 0, s>>>(
-            data, n - 1, dim, k, queries, nq, 1, KCAP, by_slot ? 1 : 0, 0, ci.get(), cd.get(), out_idx, out_dist,
-            out_dist64, redo.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(), TC_REL_BOUND,
-            tc_err.get());
+            data, n - 1, dim, k, queries, nq, 1, KCAP, by_slot ? 1 : 0, 0, 0, ci.get(), cd.get(), out_idx, out_dist,
+            out_dist64, redo.get(), redo_kth.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(),
+            TC_REL_BOUND, tc_err.get());
     }
     UMAPB_LAUNCH_CHECK();
     int32_t nredo = 0;
@@ -469,14 +609,7 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
     last_knn_redo_count() = nredo;
     last_knn_tc_error() = tc ? static_cast<double>(bits_to_float(err_bits)) : 0.0;
     if (nredo > 0) {
-        // exact FP64 search for the uncertain queries (same output rows)
-        if (k + 8 <= 32) {
-            run_f64<float, 32>(data, n, dim, k, redo.get(), nredo, out_idx, out_dist, out_dist64, s);
-        } else if (k + 8 <= 64) {
-            run_f64<float, 64>(data, n, dim, k, redo.get(), nredo, out_idx, out_dist, out_dist64, s);
-        } else {
-            run_f64<float, 128>(data, n, dim, k, redo.get(), nredo, out_idx, out_dist, out_dist64, s);
-        }
+        run_within(data, n, dim, k, redo.get(), nredo, redo_kth.get(), 0, out_idx, out_dist, out_dist64, s);
     }
 }
 
@@ -524,8 +657,8 @@ void run_f32_batched(const float* data, const std::vector<int32_t>& inst, int32_
     DevArray<unsigned int> tc_err(1, s);
     tc_err.zero(s);
     knn_rescore_kernel<per_lane<KCAP>()><<<rescore_grid(n), RESCORE_WARPS * 32, 0, s>>>(
-        data, n - 1, dim, k, nullptr, n, 1, KCAP, 0, 0, ci.get(), cd.get(), out_idx, out_dist, nullptr, redo.get(),
-        redo_count.get(), norms.get(), norm_max.get(), TC_REL_BOUND, tc_err.get());
+        data, n - 1, dim, k, nullptr, n, 1, KCAP, 0, 0, 0, ci.get(), cd.get(), out_idx, out_dist, nullptr, redo.get(),
+        nullptr, redo_count.get(), norms.get(), norm_max.get(), TC_REL_BOUND, tc_err.get());
     UMAPB_LAUNCH_CHECK();
     int32_t nredo = 0;
     unsigned int err_bits = 0;
@@ -694,11 +827,12 @@ void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int
         UMAPB_LAUNCH_CHECK();
     }
     DevArray<int32_t> redo(nq, s), redo_count(1, s);
+    DevArray<double> redo_kth(nq, s);
     redo_count.zero(s);
     auto rescore = [&](auto per) {
         knn_rescore_kernel<decltype(per)::value><<<rescore_grid(nq), RESCORE_WARPS * 32, 0, s>>>(
-            data, nref, dim, k, rows, nq, tc ? lists : 1, KCAP, 1, 1, ci.get(), cd.get(), out_idx, out_dist, nullptr,
-            redo.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(), TC_REL_BOUND, nullptr);
+            data, nref, dim, k, rows, nq, tc ? lists : 1, KCAP, 1, 1, 0, ci.get(), cd.get(), out_idx, out_dist, nullptr,
+            redo.get(), redo_kth.get(), redo_count.get(), tc ? norms.get() : nullptr, norm_max.get(), TC_REL_BOUND, nullptr);
         UMAPB_LAUNCH_CHECK();
     };
     if (tc && lists * KCAP > 32 * per_lane<KCAP>()) rescore(std::integral_constant<int, 4>());
@@ -711,9 +845,7 @@ void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int
         DevArray<int32_t> redo_rows(nredo, s);
         add_offset_kernel<<<grid_for(nredo, 256), 256, 0, s>>>(nredo, redo.get(), nref, redo_rows.get());
         UMAPB_LAUNCH_CHECK();
-        if (k + 8 <= 32) run_f64<float, 32>(data, nref, dim, k, redo_rows.get(), nredo, out_idx, out_dist, nullptr, s, redo.get());
-        else if (k + 8 <= 64) run_f64<float, 64>(data, nref, dim, k, redo_rows.get(), nredo, out_idx, out_dist, nullptr, s, redo.get());
-        else run_f64<float, 128>(data, nref, dim, k, redo_rows.get(), nredo, out_idx, out_dist, nullptr, s, redo.get());
+        run_within(data, nref, dim, k, redo_rows.get(), nredo, redo_kth.get(), nref, out_idx, out_dist, nullptr, s);
     }
 }
 
