@@ -100,3 +100,20 @@ def test_far_from_origin_costs_little(umap):
             best = min(best, time.perf_counter() - t)
         seconds.append(best)
     assert seconds[1] <= 3 * seconds[0], seconds
+
+
+@pytest.mark.parametrize("n,dim,k,few", [(150, 2, 25, True), (1075, 2, 30, True), (1076, 2, 30, False), (499, 50, 56, True),
+                                         (500, 50, 56, False), (150, 2, 57, False), (60, 100, 30, False)])
+def test_few_points_take_the_short_search(umap, monkeypatch, n, dim, k, few):
+    """Few points with 25 to 56 neighbours are searched as without tensor cores (the same launches)."""
+    X = oracle.gaussian_mixture(n, dim, 4, 3.0, seed=n, dtype=np.float32)
+    launches = []
+    for cores in (None, "0"):
+        if cores:
+            monkeypatch.setenv("UMAPB_KNN_TENSOR_CORES", cores)
+        umap.knn(X, k)
+        before = umap.lib().umapb_launch_count()
+        result = umap.knn(X, k)
+        launches.append(umap.lib().umapb_launch_count() - before)
+        check(*result, *oracle.knn(X, k))
+    assert (launches[0] == launches[1]) == few, launches

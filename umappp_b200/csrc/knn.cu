@@ -515,6 +515,14 @@ void shard_row_range(int32_t n, KnnShard shard, int32_t& lo, int32_t& hi) {
     hi = static_cast<int32_t>(static_cast<int64_t>(n) * (shard.index + 1) / shard.count);
 }
 
+// Few points with 25 to 56 neighbours: the CUDA-core search, whose cost grows
+// with n x dim, against the tensor cores' fixed one (tree, operands, two passes).
+// ms, CUDA / tensor cores, 30 neighbours: 150 x 2 points 0.25 / 0.41, 600 x 2 0.72 /
+// 0.66, 1,000 x 2 0.83 / 0.89; 300 x 20 0.47 / 0.66, 800 x 20 0.90 / 0.98; 300 x 50 0.59 /
+// 0.66, 500 x 50 0.84 / 0.77; 128 x 100 0.57 / 0.51.  (Beyond 56 neighbours, with
+// lists of 128, the tensor cores are ahead from 100 points on: 0.50 / 0.47 for 150 x 2.)
+bool few_points(int32_t n, int32_t dim, int kcap) { return kcap == 64 && n < 1100 - 12 * static_cast<int64_t>(dim); }
+
 // With a shard (count > 1) the search covers only the shard's queries, whose
 // data rows go to *rows (*nrows of them); out_idx / out_dist are written at
 // those rows only.
@@ -525,7 +533,7 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
     const bool sharded = shard.count > 1;
     DevArray<float> norms;
     DevArray<unsigned int> norm_max(1, s);
-    bool tc = use_tensor_cores() && knn_tc_supported(dim, KCAP);
+    bool tc = use_tensor_cores() && knn_tc_supported(dim, KCAP) && !few_points(n, dim, KCAP);
     // candidates: by data row (tensor-core search, unsharded brute force) or by
     // slot of the shard's row list (sharded brute force)
     DevArray<int32_t> ci;
