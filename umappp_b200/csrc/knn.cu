@@ -356,6 +356,15 @@ void run_f64(const T* data, int32_t n, int32_t dim, int32_t k, const int32_t* qu
     UMAPB_LAUNCH_CHECK();
 }
 
+// FP64 search of queries whose lists are as long as k asks for.
+void run_f64_lists(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
+                   const int32_t* out_rows, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
+    if (k <= 16) run_f64<float, 16>(data, n, dim, k, queries, nq, out_idx, out_dist, out_dist64, s, out_rows);
+    else if (k <= 32) run_f64<float, 32>(data, n, dim, k, queries, nq, out_idx, out_dist, out_dist64, s, out_rows);
+    else if (k <= 64) run_f64<float, 64>(data, n, dim, k, queries, nq, out_idx, out_dist, out_dist64, s, out_rows);
+    else run_f64<float, 128>(data, n, dim, k, queries, nq, out_idx, out_dist, out_dist64, s, out_rows);
+}
+
 // ---- uncertain queries ----
 // A query whose candidates leave its k-th neighbour open: what they do tell is a
 // distance within which k points lie (kth).  All points that may be that near are
@@ -436,27 +445,32 @@ __global__ void knn_crowded_kernel(int32_t nq, int32_t places, const int32_t* __
     }
 }
 
-// Exact search of 'nq' queries (data rows) among the data rows [0, n), k of
-// which are known to lie within kth; results to rows query - row0.
-template <int LIST>
-void run_within_lists(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
-                const double* kth, int32_t row0, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
-    int32_t batch = std::min(nq, WITHIN_PLACES / LIST);
-    DevArray<int32_t> list, count, crowded, rows, num(1, s);
-    DevArray<float> unused;   // the rescoring's FP32 distances
-    for (;; batch = (batch + 3) / 4) {
-        try {
-            list.allocate(static_cast<size_t>(batch) * LIST, s);
-            unused.allocate(static_cast<size_t>(batch) * LIST, s);
-            count.allocate(batch, s);
-            crowded.allocate(batch, s);
-            rows.allocate(batch, s);
-            break;
-        } catch (const Error& e) {
-            list.release();
-            if (e.code != UMAPB_ERR_OOM || batch <= KNN_BLOCK) throw;
-        }
+// An array that a search does without where memory is short (false).
+template <typename T>
+bool allocate_if_possible(DevArray<T>& a, size_t n, cudaStream_t s) {
+    try {
+        a.allocate(n, s);
+    } catch (const Error& e) {
+        if (e.code != UMAPB_ERR_OOM) throw;
+        return false;
     }
+    return true;
+}
+
+// Exact search of 'nq' queries (data rows) among the data rows [0, n), k of
+// which are known to lie within kth; results to rows query - row0.  False,
+// with nothing done, where there is no memory for it.
+template <int LIST>
+bool run_within_lists(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
+                const double* kth, int32_t row0, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
+    const int32_t batch = std::min(nq, WITHIN_PLACES / LIST);
+    DevArray<int32_t> list, count, crowded, rows, num;
+    DevArray<float> unused;   // the rescoring's FP32 distances
+    const size_t places = static_cast<size_t>(batch) * LIST;
+    if (!allocate_if_possible(list, places, s) || !allocate_if_possible(unused, places, s) ||
+        !allocate_if_possible(count, batch, s) || !allocate_if_possible(crowded, batch, s) ||
+        !allocate_if_possible(rows, batch, s) || !allocate_if_possible(num, 1, s))
+        return false;
     for (int32_t at = 0; at < nq; at += batch) {
         const int32_t m = std::min(batch, nq - at);
         const int32_t* q = queries + at;
@@ -479,17 +493,19 @@ void run_within_lists(const float* data, int32_t n, int32_t dim, int32_t k, cons
         int32_t nc = 0;
         UMAPB_CUDA(cudaMemcpyAsync(&nc, num.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         UMAPB_SYNC(s);
-        if (nc == 0) continue;
-        if (k <= 16) run_f64<float, 16>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
-        else if (k <= 32) run_f64<float, 32>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
-        else if (k <= 64) run_f64<float, 64>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
-        else run_f64<float, 128>(data, n, dim, k, crowded.get(), nc, out_idx, out_dist, out_dist64, s, rows.get());
+        if (nc > 0) run_f64_lists(data, n, dim, k, crowded.get(), nc, rows.get(), out_idx, out_dist, out_dist64, s);
     }
+    return true;
 }
-void run_within(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
-                const double* kth, int32_t row0, int32_t* out_idx, float* out_dist, double* out_dist64, cudaStream_t s) {
-    if (k <= 56) run_within_lists<128>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s);
-    else run_within_lists<256>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s);
+
+// The uncertain queries of a search: kth (null: unknown) as above; results to
+// rows out_rows[i], which are queries[i] - row0 (null: queries[i]).
+void search_again(const float* data, int32_t n, int32_t dim, int32_t k, const int32_t* queries, int32_t nq,
+                  const double* kth, int32_t row0, const int32_t* out_rows, int32_t* out_idx, float* out_dist,
+                  double* out_dist64, cudaStream_t s) {
+    const bool done = kth && (k <= 56 ? run_within_lists<128>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s)
+                                      : run_within_lists<256>(data, n, dim, k, queries, nq, kth, row0, out_idx, out_dist, out_dist64, s));
+    if (!done) run_f64_lists(data, n, dim, k, queries, nq, out_rows, out_idx, out_dist, out_dist64, s);
 }
 
 __global__ void norm_max_kernel(int32_t n, const float* __restrict__ norms, unsigned int* __restrict__ out) {
@@ -542,22 +558,27 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
     int32_t nq = n;
     const int32_t* queries = nullptr;
     bool by_slot = false;
+    if (sharded) *nrows = -1;
     if (tc) {
-        ci.allocate(static_cast<size_t>(n) * KCAP, s);
-        cd.allocate(static_cast<size_t>(n) * KCAP, s);
-        const int32_t n_pad = ((n + 127) / 128) * 128;
-        norms.allocate(n_pad, s);
         DevArray<int> err(1, s);
         err.zero(s);
         // unsharded: the rows in tree order, so that the rescoring walks the
         // queries with nearby ones together (their candidates share L2 lines)
         try {
+            ci.allocate(static_cast<size_t>(n) * KCAP, s);
+            cd.allocate(static_cast<size_t>(n) * KCAP, s);
+            norms.allocate(((n + 127) / 128) * 128, s);
             tc = knn_tc_candidates(data, n, dim, KCAP, ci.get(), cd.get(), norms.get(), err.get(), s, shard, rows, nrows,
                                    sharded ? nullptr : &tree_rows);
         } catch (const Error& e) {
-            // beyond 32 candidates the CUDA-core search, which needs no operands, does where memory is short
-            if (e.code != UMAPB_ERR_OOM || KCAP <= 32) throw;
+            // Beyond 32 candidates the CUDA-core search, which needs no operands, does
+            // where memory is short: of the shard's rows in the tree, the same that
+            // another process finds with more memory, or not at all.
+            if (e.code != UMAPB_ERR_OOM || KCAP <= 32 || (sharded && *nrows < 0)) throw;
             tc = false;
+            ci.release();
+            cd.release();
+            norms.release();
         }
         int h_err = 0;
         UMAPB_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -576,16 +597,18 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
         }
     }
     if (!tc) {
-        if (sharded) {   // contiguous data rows, CUDA-core candidates by slot
-            int32_t lo, hi;
-            shard_row_range(n, shard, lo, hi);
-            *nrows = hi - lo;
-            rows->allocate(std::max<int32_t>(hi - lo, 1), s);
-            if (hi > lo) {
-                iota_kernel<<<grid_for(hi - lo, 256), 256, 0, s>>>(hi - lo, lo, rows->get());
-                UMAPB_LAUNCH_CHECK();
+        if (sharded) {   // CUDA-core candidates by slot
+            if (*nrows < 0) {   // contiguous data rows
+                int32_t lo, hi;
+                shard_row_range(n, shard, lo, hi);
+                *nrows = hi - lo;
+                rows->allocate(std::max<int32_t>(hi - lo, 1), s);
+                if (hi > lo) {
+                    iota_kernel<<<grid_for(hi - lo, 256), 256, 0, s>>>(hi - lo, lo, rows->get());
+                    UMAPB_LAUNCH_CHECK();
+                }
             }
-            nq = hi - lo;
+            nq = *nrows;
             queries = rows->get();
             by_slot = true;
         }
@@ -598,7 +621,8 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
         }
     }
     DevArray<int32_t> redo(std::max(nq, 1), s), redo_count(1, s);
-    DevArray<double> redo_kth(std::max(nq, 1), s);
+    DevArray<double> redo_kth;
+    allocate_if_possible(redo_kth, std::max(nq, 1), s);
     redo_count.zero(s);
     DevArray<unsigned int> tc_err(1, s);
     tc_err.zero(s);
@@ -617,7 +641,7 @@ void run_f32(const float* data, int32_t n, int32_t dim, int32_t k, int32_t* out_
     last_knn_redo_count() = nredo;
     last_knn_tc_error() = tc ? static_cast<double>(bits_to_float(err_bits)) : 0.0;
     if (nredo > 0) {
-        run_within(data, n, dim, k, redo.get(), nredo, redo_kth.get(), 0, out_idx, out_dist, out_dist64, s);
+        search_again(data, n, dim, k, redo.get(), nredo, redo_kth.get(), 0, nullptr, out_idx, out_dist, out_dist64, s);
     }
 }
 
@@ -802,20 +826,25 @@ template <int KCAP>
 void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int32_t k, const int32_t* rows,
                    int32_t* out_idx, float* out_dist, cudaStream_t s) {
     const int lists = query_lists(nref, nq, KCAP);
-    DevArray<int32_t> ci(static_cast<size_t>(nq) * lists * KCAP, s);
-    DevArray<float> cd(static_cast<size_t>(nq) * lists * KCAP, s);
+    DevArray<int32_t> ci;
+    DevArray<float> cd;
     DevArray<float> norms;
     DevArray<unsigned int> norm_max(1, s);
     bool tc = use_tensor_cores() && lists > 0 && knn_tc_supported(dim, KCAP);
     if (tc) {
-        norms.allocate(static_cast<size_t>(nref) + nq, s);
         DevArray<int> err(1, s);
         err.zero(s);
         try {
+            ci.allocate(static_cast<size_t>(nq) * lists * KCAP, s);
+            cd.allocate(static_cast<size_t>(nq) * lists * KCAP, s);
+            norms.allocate(static_cast<size_t>(nref) + nq, s);
             tc = knn_tc_query_candidates(data, nref, nq, dim, KCAP, lists, ci.get(), cd.get(), norms.get(), err.get(), s);
         } catch (const Error& e) {
-            if (e.code != UMAPB_ERR_OOM) throw;   // the CUDA-core search needs no operands
+            if (e.code != UMAPB_ERR_OOM) throw;   // the CUDA-core search needs no operands, and one list
             tc = false;
+            ci.release();
+            cd.release();
+            norms.release();
         }
         int h_err = 0;
         UMAPB_CUDA(cudaMemcpyAsync(&h_err, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -835,7 +864,8 @@ void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int
         UMAPB_LAUNCH_CHECK();
     }
     DevArray<int32_t> redo(nq, s), redo_count(1, s);
-    DevArray<double> redo_kth(nq, s);
+    DevArray<double> redo_kth;
+    allocate_if_possible(redo_kth, nq, s);
     redo_count.zero(s);
     auto rescore = [&](auto per) {
         knn_rescore_kernel<decltype(per)::value><<<rescore_grid(nq), RESCORE_WARPS * 32, 0, s>>>(
@@ -853,7 +883,8 @@ void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int
         DevArray<int32_t> redo_rows(nredo, s);
         add_offset_kernel<<<grid_for(nredo, 256), 256, 0, s>>>(nredo, redo.get(), nref, redo_rows.get());
         UMAPB_LAUNCH_CHECK();
-        run_within(data, nref, dim, k, redo_rows.get(), nredo, redo_kth.get(), nref, out_idx, out_dist, nullptr, s);
+        search_again(data, nref, dim, k, redo_rows.get(), nredo, redo_kth.get(), nref, redo.get(), out_idx, out_dist,
+                     nullptr, s);
     }
 }
 
