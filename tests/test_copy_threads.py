@@ -19,3 +19,9 @@ def program(tmp_path_factory):
 @pytest.mark.parametrize("first_job", [0, 2 ** 24 - 3])   # the job's number has 24 bits
 def test_copies(program, helpers, first_job):
     assert subprocess.run([program, "jobs", str(helpers), str(first_job)], timeout=30).returncode == 0
+
+
+def test_helpers_sleep_while_a_copy_waits(program):
+    """Three helpers that kept asking for work would take 1.5 s of processor time in half a second."""
+    r = subprocess.run([program, "idle"], capture_output=True, text=True, timeout=30)
+    assert r.returncode == 0 and float(r.stdout) <= 0.15

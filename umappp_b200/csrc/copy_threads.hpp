@@ -70,10 +70,12 @@ private:
     void serve() {
         uint64_t done = state_.load(std::memory_order_acquire) >> JOB;   // the last job seen
         while (true) {
-            // awake between the jobs of one copy, and shortly after it (a call copies several arrays)
+            // Awake between the jobs of one copy, which the bus paces (30 to 100 us), and
+            // shortly after it (a call copies several arrays) -- not while a copy waits
+            // for whatever is before it on its stream.
             int spin = 0;
             uint64_t job = state_.load(std::memory_order_acquire) >> JOB;
-            while (job == done && (busy.load(std::memory_order_relaxed) || ++spin < 100)) {
+            while (job == done && ++spin < (busy.load(std::memory_order_relaxed) ? 1000 : 100)) {
                 std::this_thread::yield();
                 job = state_.load(std::memory_order_acquire) >> JOB;
             }
