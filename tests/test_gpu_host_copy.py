@@ -43,3 +43,30 @@ def test_round_trips_at_once(umap):
     for t in threads:
         t.join()
     assert not failures
+
+
+# pieces of half a MiB below 12 MiB, of one from there on; eight slots
+@pytest.mark.parametrize("nbytes", [MIB + MIB // 2, MIB + MIB // 2 + 4, 4 * MIB + 4, 4 * MIB + MIB // 2 + 8, 12 * MIB - 4,
+                                    12 * MIB, 12 * MIB + 4, 16 * MIB + 4])
+def test_round_trip_in_pieces(umap, nbytes):
+    for seed in range(3):
+        round_trip(umap, nbytes // 4, seed)
+
+
+@pytest.mark.parametrize("nbytes", [MIB, 5 * MIB, 8 * MIB - 4, 8 * MIB])
+def test_into_untouched_pages(umap, nbytes):
+    """Search results into arrays whose pages nobody has written yet, or the middle one only."""
+    import mmap
+
+    X = np.random.default_rng(1).normal(size=(nbytes // 40, 3)).astype(np.float32)
+    want = umap.knn(X, 10)
+    for touch in (False, True):
+        out = []
+        for t, a in ((np.int32, want[0]), (np.float32, want[1])):
+            m = np.frombuffer(mmap.mmap(-1, a.nbytes + 4096), dtype=t)[:a.size]
+            if touch:
+                m[a.size // 2] = 7
+            out.append(m)
+        umap._lib.check(umap.lib().umapb_knn(0, 3, len(X), X.ctypes.data, 10, out[0].ctypes.data, out[1].ctypes.data))
+        assert np.array_equal(out[0].reshape(want[0].shape), want[0])
+        assert np.array_equal(out[1].reshape(want[1].shape), want[1])

@@ -16,7 +16,7 @@ namespace umapb {
 // memcpy by several threads.  One job at a time (callers hold 'owner').
 class CopyThreads {
 public:
-    static constexpr size_t PART_BYTES = size_t(128) << 10;
+    static constexpr size_t PART_BYTES = size_t(64) << 10;
     // Beside the caller: 'helpers' threads, started with the first copy.  first_job: for tests.
     explicit CopyThreads(int helpers, uint64_t first_job = 0) : helpers_(helpers), state_(first_job << JOB) {}
     std::mutex owner;

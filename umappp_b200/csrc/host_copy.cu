@@ -9,9 +9,12 @@
 // graph of 2 million edges (18 MB) 1.0 instead of 1.3.
 //
 // The slots of a device are one copy's at a time; another thread that copies
-// meanwhile takes the runtime's way.  They and the threads, which sleep
+// meanwhile takes the runtime's way, as do downloads of few MB into pages that
+// are there.  They and the threads, which sleep
 // between copies, last for the process: 8 MiB pinned per device used.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <map>
@@ -26,8 +29,17 @@ namespace umapb {
 namespace {
 
 constexpr size_t COPY_MIN = size_t(1) << 20;
-constexpr size_t SLOT_BYTES = size_t(2) << 20;
-constexpr int SLOTS = 4;
+constexpr size_t SLOT_BYTES = size_t(1) << 20;
+constexpr int SLOTS = 8;
+
+// Bytes moved at a time.  The bus moves a slot only once it is full, and the
+// helpers take some 100 us to wake, so a copy of few MB goes in pieces that the
+// caller fills alone meanwhile; a large one pays more for each piece than it gains.
+// us after 0.3 ms without copies, up / down, in pieces of 512 KB | 1 MB | four of 2 MB
+// | the runtime's copy: 2 MB 128 / 166 | 169 / 223 | 289 / 366 | 209 / 144; 8 MB 411 / 359 |
+// 448 / 405 | 639 / 410 | 785 / 503; 32 MB 1625 / 1252 | 1460 / 1150 | 1493 / 1060 |
+// 3009 / 1957.  Into fresh pages 2 MB take 356 us in pieces of 512 KB (934 by the runtime).
+size_t piece_bytes(size_t bytes) { return bytes < (size_t(12) << 20) ? SLOT_BYTES / 2 : SLOT_BYTES; }
 constexpr int MAX_THREADS = 4;   // the caller among them
 
 CopyThreads& copy_threads() {
@@ -73,10 +85,27 @@ Memory memory_of(const void* p) {
          : attr.type == cudaMemoryTypeUnregistered ? Memory::pageable : Memory::other;
 }
 
+// Below WARM_MIN bytes the runtime's copy is faster into pages that are there
+// already (us, 0.3 ms after the last copy, slots | runtime: 2 MB 179 | 128, 4 MB 228 | 227,
+// 8 MB 395 | 422), and far slower into untouched ones (2 MB 380 | 922).
+constexpr size_t WARM_MIN = size_t(8) << 20;
+
+// Whether an array has pages that were never touched (three of them are asked for).
+bool untouched(const char* p, size_t bytes) {
+    const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+    for (const size_t at : {size_t(0), bytes / 2, bytes - 1}) {
+        unsigned char there = 1;
+        void* q = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + at) / page * page);
+        if (mincore(q, 1, &there) == 0 && !(there & 1)) return true;
+    }
+    return false;
+}
+
 void to_device(Slots& st, char* dst, const char* src, size_t bytes, cudaStream_t s) {
+    const size_t piece = piece_bytes(bytes);
     int i = 0;
-    for (size_t at = 0; at < bytes; at += SLOT_BYTES, i = (i + 1) % SLOTS) {
-        const size_t len = std::min(SLOT_BYTES, bytes - at);
+    for (size_t at = 0; at < bytes; at += piece, i = (i + 1) % SLOTS) {
+        const size_t len = std::min(piece, bytes - at);
         UMAPB_CUDA(cudaEventSynchronize(st.moved[i]));
         copy_threads().copy(st.slot[i], src + at, len);
         UMAPB_CUDA(cudaMemcpyAsync(dst + at, st.slot[i], len, cudaMemcpyHostToDevice, s));
@@ -85,19 +114,20 @@ void to_device(Slots& st, char* dst, const char* src, size_t bytes, cudaStream_t
 }
 
 void to_host(Slots& st, char* dst, const char* src, size_t bytes, cudaStream_t s) {
-    const size_t chunks = (bytes + SLOT_BYTES - 1) / SLOT_BYTES;
+    const size_t piece = piece_bytes(bytes);
+    const size_t pieces = (bytes + piece - 1) / piece;
     auto move = [&](size_t c) {
-        const size_t at = c * SLOT_BYTES;
-        UMAPB_CUDA(cudaMemcpyAsync(st.slot[c % SLOTS], src + at, std::min(SLOT_BYTES, bytes - at), cudaMemcpyDeviceToHost, s));
+        const size_t at = c * piece;
+        UMAPB_CUDA(cudaMemcpyAsync(st.slot[c % SLOTS], src + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, s));
         UMAPB_CUDA(cudaEventRecord(st.moved[c % SLOTS], s));
     };
     for (int i = 0; i < SLOTS; ++i) UMAPB_CUDA(cudaEventSynchronize(st.moved[i]));   // free of the copy before
-    for (size_t c = 0; c < std::min<size_t>(chunks, SLOTS); ++c) move(c);
-    for (size_t c = 0; c < chunks; ++c) {
-        const size_t at = c * SLOT_BYTES;
+    for (size_t c = 0; c < std::min<size_t>(pieces, SLOTS); ++c) move(c);
+    for (size_t c = 0; c < pieces; ++c) {
+        const size_t at = c * piece;
         UMAPB_CUDA(cudaEventSynchronize(st.moved[c % SLOTS]));
-        copy_threads().copy(dst + at, st.slot[c % SLOTS], std::min(SLOT_BYTES, bytes - at));
-        if (c + SLOTS < chunks) move(c + SLOTS);
+        copy_threads().copy(dst + at, st.slot[c % SLOTS], std::min(piece, bytes - at));
+        if (c + SLOTS < pieces) move(c + SLOTS);
     }
 }
 
@@ -109,7 +139,7 @@ void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s) {
         const Memory to = memory_of(dst), from = memory_of(src);
         const bool up = to == Memory::device && from == Memory::pageable;
         const bool down = to == Memory::pageable && from == Memory::device;
-        if (up || down) {
+        if (up || (down && (bytes >= WARM_MIN || untouched(static_cast<const char*>(dst), bytes)))) {
             std::unique_lock<std::mutex> lock(copy_threads().owner, std::try_to_lock);
             Slots* st = lock.owns_lock() ? device_slots() : nullptr;
             if (st) {
