@@ -269,6 +269,9 @@ Context& thread_context();                 // defined in capi.cu
 void set_last_error(const std::string& m);  // message for umapb_last_error() on this thread
 void check_device_status(Context& ctx);     // reads and clears the status word; throws on error
 
+int current_device();   // memory.cu
+int sm_count();         // of the current device
+
 inline unsigned grid_for(size_t work, unsigned block, unsigned max_blocks = 148u * 64u) {
     size_t g = (work + block - 1) / block;
     if (g < 1) g = 1;

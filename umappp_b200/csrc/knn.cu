@@ -479,7 +479,7 @@ bool run_within_lists(const float* data, int32_t n, int32_t dim, int32_t k, cons
         num.zero(s);
         // stretches so that the device is filled four times over
         const int32_t blocks = (m + KNN_BLOCK - 1) / KNN_BLOCK, tiles = (n - 1) / PT + 1;
-        const int32_t parts = std::min(tiles, std::max(1, 4 * 4 * 148 / blocks));
+        const int32_t parts = std::min(tiles, std::max(1, 4 * 4 * sm_count() / blocks));
         const int32_t stretch = (tiles + parts - 1) / parts * PT;
         knn_within_kernel<LIST><<<dim3(blocks, (tiles - 1) / (stretch / PT) + 1), KNN_BLOCK, 0, s>>>(data, n, dim, q, m, kth + at,
                                                                                          stretch, list.get(), count.get());
@@ -807,7 +807,7 @@ static int query_lists(int32_t nref, int32_t nq, int kcap) {
     if (nref < 1024) return 0;
     const int64_t tiles = (static_cast<int64_t>(nq) + 127) / 128;
     int lists = 1;
-    while (lists < 4 && 2 * lists * kcap <= 128 && tiles * lists < 2 * 148) lists *= 2;
+    while (lists < 4 && 2 * lists * kcap <= 128 && tiles * lists < 2 * sm_count()) lists *= 2;
     return lists;
 }
 

@@ -23,8 +23,25 @@
 #include <vector>
 
 #include "common.cuh"
+#include "per_device.hpp"
 
 namespace umapb {
+
+int current_device() {
+    int d = 0;
+    cudaGetDevice(&d);
+    return d;
+}
+
+int sm_count() {
+    static PerDevice count;
+    const int dev = current_device();
+    return static_cast<int>(count.get(dev, [&] {
+        int c = 0;
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+        return int64_t(c > 0 ? c : 148);
+    }));
+}
 
 namespace {
 
@@ -59,12 +76,6 @@ size_t bucket(size_t bytes) {
         return b;
     }
     return (bytes + 2 * MiB - 1) / (2 * MiB) * (2 * MiB);
-}
-
-int current_device() {
-    int d = 0;
-    cudaGetDevice(&d);
-    return d;
 }
 
 // Hands every cached block back to the device pool (cache lock held).

@@ -30,6 +30,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "per_device.hpp"
 #include "pow_pos.cuh"
 #include "stages.cuh"
 #include "umap_grad.cuh"
@@ -979,17 +980,6 @@ size_t window_bytes() {
 // Calls of at most this many epochs have their lists read ahead (SgdEngine::run).
 constexpr int FEW_EPOCHS = 8;
 
-int sm_count() {
-    static int count = 0;
-    if (count == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-        if (count <= 0) count = 148;
-    }
-    return count;
-}
-
 // Rows in flight at once: at most n / window_div (a sliding window over the
 // claim order), so that few rows run beside their neighbours with positions
 // read before those neighbours' updates, in steps of 256; small layouts take
@@ -1134,6 +1124,7 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
     stream.num_inst = num_inst_;
     const T lr = static_cast<T>(learning_rate);
     const bool check = check_schedule();
+    const int device = current_device();
     const int64_t rows = rows_in_flight(n, window_div);
     // Points are read and added to as vectors of up to 16 bytes: a layout of
     // three dimensions, and an array that is not aligned to them, is worked on
@@ -1258,13 +1249,17 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
                     constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
                     const RowTask* tasks = lists_.tasks(buffer) + static_cast<size_t>(e - w.first) * n;
                     if (relay_rows(rows)) {
-                        static const int64_t resident = resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS);
+                        static PerDevice known;
+                        const int64_t resident = known.get(
+                            device, [] { return resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS); });
                         const int share = relay_share<G>(rows);
                         const int64_t blocks = std::min((rows + share - 1) / share, resident);
                         sgd_relay_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), 32 * RELAY_WARPS, 0, es>>>(
                             tasks, n, lists_.list(buffer), Yp, stride, counters.get() + (e - first), share, p);
                     } else {
-                        static const int64_t resident = resident_blocks(sgd_rows_kernel<T, NC, G, CH>, ROW_BLOCK);
+                        static PerDevice known;
+                        const int64_t resident = known.get(
+                            device, [] { return resident_blocks(sgd_rows_kernel<T, NC, G, CH>, ROW_BLOCK); });
                         const int64_t blocks = std::min((rows * G + ROW_BLOCK - 1) / ROW_BLOCK, resident);
                         sgd_rows_kernel<T, NC, G, CH><<<static_cast<unsigned>(blocks), ROW_BLOCK, 0, es>>>(
                             tasks, n, lists_.list(buffer), Yp, stride, counters.get() + (e - first), p);

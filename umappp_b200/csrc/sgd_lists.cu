@@ -414,11 +414,8 @@ GenArgs<T> gen_args(const DeviceEpochs<T>& ep, const int32_t* seg_row, int64_t n
 // Blocks for nseg segments: as many as are resident at once, each taking
 // segment after segment.
 unsigned gen_grid(int64_t nseg, bool beside_epochs) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int per_sm = beside_epochs ? GEN_BLOCKS_BESIDE : GEN_BLOCKS;
-    return static_cast<unsigned>(std::min<int64_t>((nseg + GEN_WARPS - 1) / GEN_WARPS, int64_t(sms) * per_sm));
+    return static_cast<unsigned>(std::min<int64_t>((nseg + GEN_WARPS - 1) / GEN_WARPS, int64_t(sm_count()) * per_sm));
 }
 
 }  // namespace

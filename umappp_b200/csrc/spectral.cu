@@ -389,7 +389,7 @@ struct LanczosDevice {
         nblk = static_cast<int>(std::min<int64_t>((n + 1023) / 1024, 256));
         partial.allocate(nblk, s);
         tmp.allocate(static_cast<size_t>(n) * (ncv + 1), s);
-        steps_blk = static_cast<int>(std::min<int64_t>((n + STEP_WARPS - 1) / STEP_WARPS, 2 * 148));
+        steps_blk = static_cast<int>(std::min<int64_t>((n + STEP_WARPS - 1) / STEP_WARPS, 2 * sm_count()));
         for (int b = 0; b < 2; ++b) {
             w[b].allocate(n, s);
             dots[b].allocate(static_cast<size_t>(steps_blk) * (ncv + 1), s);
