@@ -389,6 +389,14 @@ def run_batch(args, rank: int, world: int) -> dict | None:
 
 # --------------------------------------------------- reference on CPU ---
 
+def no_reference() -> str | None:
+    """Why the reference cannot be timed here, or None: it is compiled from its own headers, which are not part of
+    this repository."""
+    import oracle
+
+    return None if oracle.ref_available() else "the reference is not built (it needs its sources)"
+
+
 def cpu_sample(cfg: str, budget_queries: int = 1000, sub_n: int = 50_000, sgd_epochs: int = 10) -> dict:
     """Times the reference (oracle/_ref) on the host cores and scales it to the full workload:
     - kNN: the stand-in exact brute force on the full data for 'budget_queries'
@@ -569,6 +577,10 @@ def main() -> None:
                 print(json.dumps({"impl": "reference", "unavailable": "batch64 is a device-only mode without a "
                                   "reference counterpart"}), flush=True)
             return
+        if no_reference():
+            if rank == 0:
+                print(json.dumps({"impl": "reference", "unavailable": no_reference()}), flush=True)
+            return
         out = run_reference(args, rank)
         if out is not None:
             print(json.dumps(out), flush=True)
@@ -591,7 +603,7 @@ def main() -> None:
             out["precision"] = precision_study(args.config)
         if rank == 0 and out is not None:
             if world == 1 and not args.no_cpu_baseline and args.config != "batch64":
-                out["cpu_baseline"] = cpu_sample(args.config)
+                out["cpu_baseline"] = {"unavailable": no_reference()} if no_reference() else cpu_sample(args.config)
             print(json.dumps(out), flush=True)
     finally:
         if world > 1:
