@@ -97,6 +97,13 @@ def test_separate_rows_match_serial(umap, n, heads, num_dim, dtype):
     assert np.max(np.abs(Yd - Y)) <= tol
 
 
+# where relays end with more lanes per row: 1,536, 1,024 and 3,072 rows in flight
+@pytest.mark.parametrize("n,num_dim,dtype", [(12288, 20, np.float32), (12289, 20, np.float32), (8192, 20, np.float64), (8193, 40, np.float64),
+                                             (24576, 10, np.float64), (24577, 16, np.float64)])
+def test_separate_rows_where_relays_end(umap, n, num_dim, dtype):
+    test_separate_rows_match_serial(umap, n, 150, num_dim, dtype)
+
+
 @pytest.mark.parametrize("num_dim", [2, 3, 4])
 def test_unaligned_layout(umap, num_dim):
     torch = pytest.importorskip("torch")

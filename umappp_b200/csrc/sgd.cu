@@ -1006,12 +1006,23 @@ int64_t resident_blocks(K kernel, int threads) {
 }
 
 // Whether an epoch with this many rows in flight is run by relays: as long as
-// its time is the longest rows' chains rather than what the SMs issue.  100
-// epochs (whole runs, relays / single warps, 15 neighbours): 1,000 x 2 f32
-// points 3.6 / 4.7 ms, 10,000 7.8 / 10.2, 45,000 (5,632 rows in flight) 13.0 /
-// 14.8, 64,000 (8,192) 15.5 / 15.5, a batch of 91,000 (11,520) 15.9 / 13.4;
-// 30,000 x 5 f32 13.8 / 21.1, 20,000 x 2 f64 31.7 / 39.4.
-bool relay_rows(int64_t rows) { return rows <= 6144; }
+// its time is the longest rows' chains rather than what the SMs issue.  With more
+// lanes per row a warp has fewer rows, and the relays that are resident (six to
+// eight per SM) are out sooner.  ms for 15 neighbours, relays / single warps (epochs):
+//   2 x f32 (50)  45,000 points 3.55 / 4.26, 70,000 4.82 / 4.51
+//   5 x f32 (20)  45,000 1.65 / 2.48        10 x f32 (20)  45,000 2.84 / 2.91, 55,000 3.37 / 3.26
+//   40 x f32 (30) 8,000 2.46 / 3.14, 12,000 3.44 / 3.34; (20) 45,000 7.57 / 5.00
+//   2 x f64 (20)  45,000 2.84 / 4.16        5 x f64 (20)  45,000 3.84 / 4.69
+//   10 x f64 (30) 20,000 5.57 / 6.60, 36,000 8.85 / 7.96
+//   40 x f64 (30) 8,000 5.57 / 6.07, 12,000 8.05 / 6.46; (20) 45,000 18.3 / 10.3
+// (an eighth of the points are in flight up to 262,144; 8 and fewer dimensions, and
+// doubles of up to 4, would gain from relays beyond 6,144 rows: 55,000 x 5 f32 1.90 /
+// 2.54, 100,000 x 2 f64 3.41 / 4.64.)
+template <typename T, int G>
+bool relay_rows(int64_t rows) {
+    constexpr bool twice = sizeof(T) == 8;
+    return rows <= (G == 32 ? (twice ? 1024 : 1536) : G == 16 && twice ? 3072 : 6144);
+}
 
 // Rows per relay: the fewest with which RELAY_BLOCKS per SM hold all rows (a
 // relay's steps are faster with few rows, and it waits for the longest of
@@ -1248,7 +1259,7 @@ void SgdEngine<T>::run(T* Y, int num_dim, int first, int last, double a, double 
                 for_dim<T>(stride, [&](auto nc, auto g, auto ch) {
                     constexpr int NC = decltype(nc)::value, G = decltype(g)::value, CH = decltype(ch)::value;
                     const RowTask* tasks = lists_.tasks(buffer) + static_cast<size_t>(e - w.first) * n;
-                    if (relay_rows(rows)) {
+                    if (relay_rows<T, G>(rows)) {
                         static PerDevice known;
                         const int64_t resident = known.get(
                             device, [] { return resident_blocks(sgd_relay_kernel<T, NC, G, CH>, 32 * RELAY_WARPS); });
