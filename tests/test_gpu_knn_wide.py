@@ -117,3 +117,20 @@ def test_few_points_take_the_short_search(umap, monkeypatch, n, dim, k, few):
         launches.append(umap.lib().umapb_launch_count() - before)
         check(*result, *oracle.knn(X, k))
     assert (launches[0] == launches[1]) == few, launches
+
+
+@pytest.mark.parametrize("nref,dim,k,few", [(1505, 3, 8, True), (1506, 3, 8, False), (1023, 60, 5, True), (1024, 60, 5, False),
+                                            (1023, 3, 9, True), (1024, 3, 9, False)])
+def test_few_references_take_the_short_search(umap, monkeypatch, nref, dim, k, few):
+    """Queries against few references are searched as without tensor cores (the same launches)."""
+    X = oracle.gaussian_mixture(nref + 300, dim, 4, 3.0, seed=nref, dtype=np.float32)
+    launches = []
+    for cores in (None, "0"):
+        if cores:
+            monkeypatch.setenv("UMAPB_KNN_TENSOR_CORES", cores)
+        umap.knn_query(X[:nref], X[nref:], k)
+        before = umap.lib().umapb_launch_count()
+        result = umap.knn_query(X[:nref], X[nref:], k)
+        launches.append(umap.lib().umapb_launch_count() - before)
+        check(*result, *oracle.knn_query(X[:nref], X[nref:], k))
+    assert (launches[0] == launches[1]) == few, launches

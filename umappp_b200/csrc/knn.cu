@@ -802,9 +802,10 @@ template void knn_exact_shard<double>(const double*, int32_t, int32_t, int32_t, 
 // the tensor-core search to pay (10 and 500 queries, 10 and 50 dimensions: 512
 // references 0.24 and 0.27 ms against 0.18 and 0.31 on CUDA cores, 1024 0.23 and
 // 0.28 against 0.25 and 0.49; 100,000 references and 10,000 queries 2.9 against
-// 30 ms).
-static int query_lists(int32_t nref, int32_t nq, int kcap) {
-    if (nref < 1024) return 0;
+// 30 ms; with up to 8 neighbours in 3 dimensions 20,000 queries against 1,100
+// references 0.48 against 0.41, 3,000 0.53 against 0.61).
+static int query_lists(int32_t nref, int32_t nq, int32_t dim, int kcap) {
+    if (nref < 1024 || (kcap == 16 && nref < 1536 - 10 * static_cast<int64_t>(dim))) return 0;
     const int64_t tiles = (static_cast<int64_t>(nq) + 127) / 128;
     int lists = 1;
     while (lists < 4 && 2 * lists * kcap <= 128 && tiles * lists < 2 * sm_count()) lists *= 2;
@@ -825,7 +826,7 @@ __global__ void add_offset_kernel(int32_t count, const int32_t* __restrict__ src
 template <int KCAP>
 void run_query_f32(const float* data, int32_t nref, int32_t nq, int32_t dim, int32_t k, const int32_t* rows,
                    int32_t* out_idx, float* out_dist, cudaStream_t s) {
-    const int lists = query_lists(nref, nq, KCAP);
+    const int lists = query_lists(nref, nq, dim, KCAP);
     DevArray<int32_t> ci;
     DevArray<float> cd;
     DevArray<float> norms;
