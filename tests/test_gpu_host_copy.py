@@ -45,9 +45,9 @@ def test_round_trips_at_once(umap):
     assert not failures
 
 
-# pieces of half a MiB below 12 MiB, of one from there on; eight slots
-@pytest.mark.parametrize("nbytes", [MIB + MIB // 2, MIB + MIB // 2 + 4, 4 * MIB + 4, 4 * MIB + MIB // 2 + 8, 12 * MIB - 4,
-                                    12 * MIB, 12 * MIB + 4, 16 * MIB + 4])
+# pieces of half a MiB below 5 MiB, of two from there on; four slots
+@pytest.mark.parametrize("nbytes", [MIB + MIB // 2, MIB + MIB // 2 + 4, 2 * MIB + MIB // 2 + 8, 4 * MIB + 4, 5 * MIB - 4, 5 * MIB,
+                                    5 * MIB + 4, 12 * MIB + 4])
 def test_round_trip_in_pieces(umap, nbytes):
     for seed in range(3):
         round_trip(umap, nbytes // 4, seed)

@@ -9,12 +9,9 @@
 // graph of 2 million edges (18 MB) 1.0 instead of 1.3.
 //
 // The slots of a device are one copy's at a time; another thread that copies
-// meanwhile takes the runtime's way, as do downloads of few MB into pages that
-// are there.  They and the threads, which sleep
+// meanwhile takes the runtime's way.  They and the threads, which sleep
 // between copies, last for the process: 8 MiB pinned per device used.
 #include <cuda_runtime.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <algorithm>
 #include <map>
@@ -29,17 +26,20 @@ namespace umapb {
 namespace {
 
 constexpr size_t COPY_MIN = size_t(1) << 20;
-constexpr size_t SLOT_BYTES = size_t(1) << 20;
-constexpr int SLOTS = 8;
+constexpr size_t SLOT_BYTES = size_t(2) << 20;
+constexpr int SLOTS = 4;
 
-// Bytes moved at a time.  The bus moves a slot only once it is full, and the
+// Bytes moved at a time.  The bus moves a piece only once it is there, and the
 // helpers take some 100 us to wake, so a copy of few MB goes in pieces that the
-// caller fills alone meanwhile; a large one pays more for each piece than it gains.
-// us after 0.3 ms without copies, up / down, in pieces of 512 KB | 1 MB | four of 2 MB
-// | the runtime's copy: 2 MB 128 / 166 | 169 / 223 | 289 / 366 | 209 / 144; 8 MB 411 / 359 |
-// 448 / 405 | 639 / 410 | 785 / 503; 32 MB 1625 / 1252 | 1460 / 1150 | 1493 / 1060 |
-// 3009 / 1957.  Into fresh pages 2 MB take 356 us in pieces of 512 KB (934 by the runtime).
-size_t piece_bytes(size_t bytes) { return bytes < (size_t(12) << 20) ? SLOT_BYTES / 2 : SLOT_BYTES; }
+// caller fills alone meanwhile; a larger one pays more for each piece than it
+// gains.  us after 0.3 ms without copies, up / down, in pieces of 512 KB | 2 MB | the
+// runtime's copy: 2 MB 128 / 166 | 289 / 366 | 209 / 144; 4 MB 221 / 222 | 399 / 371 | 410 /
+// 263; 6.4 MB 320 / 344 | 485 / 293 | 610 / 399; 32 MB 1625 / 1252 | 1493 / 1060 | 3009 / 1957.
+// Into fresh pages, where the faults decide: 2 MB 356 | 545 | 934, 6.4 MB 845 | 773 | 2863.
+// Search of 30,011 points with 50 neighbours (3.6 MB up, twice 6 MB down into fresh
+// arrays) 5.3 ms with 512 KB throughout, 4.9 with 2 MB, 4.65 so.
+constexpr size_t PIECES_BELOW = size_t(5) << 20;
+size_t piece_bytes(size_t bytes) { return bytes < PIECES_BELOW ? SLOT_BYTES / 4 : SLOT_BYTES; }
 constexpr int MAX_THREADS = 4;   // the caller among them
 
 CopyThreads& copy_threads() {
@@ -85,22 +85,6 @@ Memory memory_of(const void* p) {
          : attr.type == cudaMemoryTypeUnregistered ? Memory::pageable : Memory::other;
 }
 
-// Below WARM_MIN bytes the runtime's copy is faster into pages that are there
-// already (us, 0.3 ms after the last copy, slots | runtime: 2 MB 179 | 128, 4 MB 228 | 227,
-// 8 MB 395 | 422), and far slower into untouched ones (2 MB 380 | 922).
-constexpr size_t WARM_MIN = size_t(8) << 20;
-
-// Whether an array has pages that were never touched (three of them are asked for).
-bool untouched(const char* p, size_t bytes) {
-    const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
-    for (const size_t at : {size_t(0), bytes / 2, bytes - 1}) {
-        unsigned char there = 1;
-        void* q = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(p) + at) / page * page);
-        if (mincore(q, 1, &there) == 0 && !(there & 1)) return true;
-    }
-    return false;
-}
-
 void to_device(Slots& st, char* dst, const char* src, size_t bytes, cudaStream_t s) {
     const size_t piece = piece_bytes(bytes);
     int i = 0;
@@ -139,7 +123,7 @@ void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s) {
         const Memory to = memory_of(dst), from = memory_of(src);
         const bool up = to == Memory::device && from == Memory::pageable;
         const bool down = to == Memory::pageable && from == Memory::device;
-        if (up || (down && (bytes >= WARM_MIN || untouched(static_cast<const char*>(dst), bytes)))) {
+        if (up || down) {
             std::unique_lock<std::mutex> lock(copy_threads().owner, std::try_to_lock);
             Slots* st = lock.owns_lock() ? device_slots() : nullptr;
             if (st) {
