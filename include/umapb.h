@@ -198,7 +198,8 @@ int umapb_initialize_prebuilt(const umapb_prebuilt* prebuilt, size_t num_dim, vo
  * Status::run(embedding, epoch_limit) (include/umappp/Status.hpp:101-128):
  * advances the layout in 'embedding' (read on entry, written on exit) from
  * epoch() to epoch_limit.  epoch_limit < 0 means num_epochs()
- * (Status::run(embedding), Status.hpp:138-140).
+ * (Status::run(embedding), Status.hpp:138-140).  A run that fails for
+ * want of device memory leaves the embedding and epoch() as they were.
  */
 int umapb_status_run(umapb_status* st, void* embedding, int epoch_limit);
 

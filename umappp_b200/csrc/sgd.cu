@@ -1040,9 +1040,10 @@ int relay_share(int64_t rows) {
 // flight has a relay of its own (up to some 5,900 points in up to 4 dimensions):
 // there are no lists to match, and longest first puts an epoch's busiest rows,
 // which pull on one another, side by side.  2,000 points, mean cross-entropy
-// against the serial reference's (some 100 x 16 runs each, standard error 0.03 %):
-// -0.49 % f64 and -0.53 % f32 sorted, -0.37 % both in the run's order, for 6 % of the
-// time (1,000 points, 500 epochs 11.8 -> 12.5 ms).
+// against the serial reference's (some 110 to 150 x 16 runs each, standard error
+// 0.02 %): -0.52 % f64 and -0.54 % f32 sorted, -0.39 % both in the run's order (as
+// before the lists: -0.40 %, 26 x 16 runs), for 6 % of the time (1,000 points, 500
+// epochs 11.8 -> 12.5 ms).
 template <typename T, int G>
 bool sort_epoch(int64_t rows) { return !(relay_rows<T, G>(rows) && relay_share<G>(rows) == 1); }
 
